@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include <cmath>
+#include <initializer_list>
 #include <string>
 #include <type_traits>
 
@@ -285,7 +286,14 @@ __global__ void k_mse(long n, int nvalid, const float *__restrict__ Y, const flo
         dY[e] = g;
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.f) atomicAdd(loss, l);
+    // one atomic per block: an atomic per warp on the one loss word serialised in L2
+    __shared__ float part[8];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = l;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) l += part[w];
+        if (l != 0.f) atomicAdd(loss, l);
+    }
 }
 
 // Adam step on FP32 master weights; refreshes the BF16 copy used by the tensor cores.
@@ -455,6 +463,431 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_infer(InferW w, long n,
     fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem);
+}
+
+// ---- training: fused forward and backward passes -------------------------------------------
+// One minibatch of the 5-layer network in four launches.  Bounds at 8192 rows (64 tiles): every
+// operand lives in L2 (about 60 MB with the saved activations), so the passes are bound by the
+// chain product -> epilogue -> product of a tile and by each SM's L1 path, not by HBM or the tensor
+// cores (7.5 GFLOP, 5 us).  Layer by layer through k_gemm an optimizer step of 8192 rows took 15.3 ms
+// (each dW product sums all its rows in one CTA, staged element by element); now 0.215 ms: k_fwd
+// 36 us, k_bwd_rows 20, k_bwd_dw 96, the rest the loss and Adam launches.
+//   k_fwd      one CTA per 128-row tile: the five layers in a row, the next layer's weights loaded
+//              beside the current product, writing the pre-activations and activations the
+//              backward pass reads (the operations of k_gemm's epilogue in its order).
+//   k_bwd_rows 64 CTAs of 128 rows at a time, the layers in reverse: G_l = dA act'(Z_l) in FP32 registers, its
+//              column sums (db), its BF16 copy as the operand of dA = G_l W_l and, for l < 4,
+//              in `work` for the weight gradients.
+//   k_bwd_dw   dW_l = G_l^T X_l, a CTA per layer and 32 input columns.  The rows are summed in order
+//              into one accumulator, as the layer-by-layer pass sums them: the tensor cores' FP32
+//              accumulation rounds towards zero, so another split of the rows moves dW by some 1e-5
+//              at 8192 rows (a split over a cluster's CTAs, summed through distributed shared
+//              memory, did), more than its own rounding.
+// The operands of a product that sums over rows (G^T, X) or over the output index (W in dA) are
+// stored as they lie in memory, [row][column], in core matrices of 8 rows x 8 columns; read as
+// "MN-major" operands the same bytes are the transposed matrix, so no transposed copy is made.
+// Core matrices lie 144 bytes apart (128 and a pad of 16): both the 16-byte stores of a row's
+// consecutive chunks and those of 8 consecutive rows then touch every bank once.  Global rows are
+// read and written by whole rows, a warp's 32 x 32 values turned through shared memory: a lane a
+// row takes 32 L1 wavefronts for 512 bytes (k_fwd 43 us, k_bwd_rows 31, k_bwd_dw 202, at 75 to 97%
+// of the L1 path).
+constexpr int kTrainThreads = 512;
+constexpr int kCore = 72;                                  // elements from core matrix to core matrix
+constexpr uint32_t kPLBO = kCore * 2, kPSBO = 16 * kPLBO;  // bytes: next 8 columns, next 8 rows
+constexpr int kPTile = 16 * 16 * kCore;                    // elements of a 128 x 128 operand
+constexpr int kTurn = 36;                                  // floats of a row in a warp's 32 x 32 turn
+constexpr size_t kRowsSmem = (size_t)3 * kPTile * 2 + (size_t)(kTrainThreads / 32) * 32 * kTurn * 4;
+constexpr int kDbParts = 256;                              // partial sums of a bias gradient
+constexpr int kDwCols = 32;                                // input columns per CTA of k_bwd_dw
+constexpr uint32_t kDwKB = (kDwCols / 8) * kPLBO;          // bytes: next 8 rows of its X columns
+constexpr int kDwRows = 256;                               // rows of a stage of k_bwd_dw
+constexpr size_t kDwStage = (kDwRows / 8) * (size_t)(kPSBO + kDwKB);
+constexpr size_t kDwSmem = 2 * kDwStage;
+constexpr uint32_t kMajA = 1u << 15, kMajB = 1u << 16;     // operand MN-major
+
+__device__ __forceinline__ void mma_bf16_d(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
+                                           uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(tmem_d),
+        "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0), "r"(0), "r"(0), "r"(0));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 b2 = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&b2);
+}
+// Element (r, k) of an operand with `chunks` 8-column chunks a row (k a multiple of 4).
+__device__ __forceinline__ int pcm_index(int r, int k, int chunks = 16) {
+    return ((r >> 3) * chunks + (k >> 3)) * kCore + ((r & 7) << 3) + (k & 7);
+}
+// 32 consecutive FP32 values of a row as BF16 at columns n0.. of an operand
+__device__ __forceinline__ void store_bf16_32(__nv_bfloat16 *t, int r, int n0, const float *v) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4 *>(&t[pcm_index(r, n0 + 8 * q)]) =
+            make_uint4(pack_bf16(v[8 * q], v[8 * q + 1]), pack_bf16(v[8 * q + 2], v[8 * q + 3]),
+                       pack_bf16(v[8 * q + 4], v[8 * q + 5]), pack_bf16(v[8 * q + 6], v[8 * q + 7]));
+}
+// A read-only 16-byte load that is issued where it stands (not sunk to its use past a barrier).
+__device__ __forceinline__ float4 ld_now(const void *p) {
+    float4 q;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w)
+                 : "l"(p));
+    return q;
+}
+// This thread's four 16-byte chunks of a 128 x 128 row-major BF16 matrix: loads, then stores.
+__device__ __forceinline__ void load_weights(float4 *q, const __nv_bfloat16 *__restrict__ W) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) q[e] = ld_now(W + (threadIdx.x + e * kTrainThreads) * 8);
+}
+__device__ __forceinline__ void put_weights(__nv_bfloat16 *dst, const float4 *q) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int c = threadIdx.x + e * kTrainThreads;
+        *reinterpret_cast<float4 *>(&dst[pcm_index(c >> 4, (c & 15) * 8)]) = q[e];
+    }
+}
+// A warp's 32 x 32 block (row lane, 32 columns in v) of a row-major array of 128 columns, whose first
+// row and column p points to; rows from `rows` on are not touched (read as 0).  t: the warp's own
+// shared memory.
+__device__ __forceinline__ void store_rows(float *__restrict__ p, const float *v, float *t, int lane,
+                                           int rows) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        *reinterpret_cast<float4 *>(t + lane * kTurn + 4 * k) =
+            make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int r = 4 * k + (lane >> 3), c = (lane & 7) * 4;
+        const float4 q = *reinterpret_cast<const float4 *>(t + r * kTurn + c);
+        if (r < rows) *reinterpret_cast<float4 *>(p + (long)r * kTile + c) = q;
+    }
+}
+__device__ __forceinline__ void load_rows(float4 *q, const float *__restrict__ p, int lane, int rows,
+                                          long pitch = kTile) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {   // rows past the end read the block's first row
+        const int r = 4 * k + (lane >> 3), c = (lane & 7) * 4;
+        if (rows > 0) q[k] = ld_now(p + (r < rows ? r : 0) * pitch + c);
+    }
+}
+__device__ __forceinline__ void turn_rows(float *v, const float4 *q, float *t, int lane, int rows) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        *reinterpret_cast<float4 *>(t + (4 * k + (lane >> 3)) * kTurn + (lane & 7) * 4) = q[k];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float4 x = *reinterpret_cast<const float4 *>(t + lane * kTurn + 4 * k);
+        v[4 * k] = x.x;
+        v[4 * k + 1] = x.y;
+        v[4 * k + 2] = x.z;
+        v[4 * k + 3] = x.w;
+    }
+    if (lane >= rows) {
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] = 0.f;
+    }
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(kTrainThreads, 1) k_fwd(InferW w, long n, const float *__restrict__ X,
+                                                          float *__restrict__ Y, float *__restrict__ acts,
+                                                          float *__restrict__ pre, int *err) {
+    extern __shared__ __align__(1024) unsigned char dsm[];
+    __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(dsm), *sW = sA + kPTile;
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tmem_base;
+    __shared__ __align__(16) float sbias[SF_MLP_LAYERS][kTile];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rb = (warp & 3) * 32, rl = rb + lane, cb = (warp >> 2) * 32;   // this warp's rows and columns
+    float *turn = reinterpret_cast<float *>(sW + 2 * kPTile) + warp * 32 * kTurn;
+    const long r0 = (long)blockIdx.x * kTile + rb;
+    const int rows = (int)(n - r0 < 32 ? n - r0 : 32);
+    if (warp == 0) tmem_alloc(&tmem_base);
+    if (tid == 0) {
+        mbar_init(&mbar);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::);
+    }
+    float v[32];
+    float4 q[8], wq[4];
+    load_weights(wq, w.W[0]);
+    load_rows(q, X + r0 * kTile + cb, lane, rows);
+    for (int e = tid; e < SF_MLP_LAYERS * kTile; e += kTrainThreads)
+        sbias[e / kTile][e % kTile] = w.b[e / kTile] ? w.b[e / kTile][e % kTile] : 0.f;
+    put_weights(sW, wq);
+    turn_rows(v, q, turn, lane, rows);
+    store_bf16_32(sA, rl, cb, v);
+    fence_before();
+    fence_proxy_async();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, trow = ((uint32_t)rb << 16) + cb;
+    bool ok = true;
+    for (int l = 0; l < SF_MLP_LAYERS; ++l) {
+        const bool last = l == SF_MLP_LAYERS - 1;
+        if (tid == 0) {
+            fence_after();
+            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sW + (l & 1) * kPTile);
+            for (int s = 0; s < kTile / 16; ++s)
+                mma_bf16(tmem, sdesc(a0 + s * 2 * kPLBO, kPLBO, kPSBO),
+                         sdesc(b0 + s * 2 * kPLBO, kPLBO, kPSBO), s > 0);
+            mma_commit(&mbar);
+        }
+        if (!last) {   // the other buffer's product (layer l - 1) is done
+            load_weights(wq, w.W[l + 1]);
+            put_weights(sW + ((l + 1) & 1) * kPTile, wq);
+        }
+        const bool done = mbar_wait(&mbar, l & 1);
+        fence_after();
+        if (__syncthreads_or(!done)) {
+            ok = false;
+            break;
+        }
+        tmem_ld32(tmem + trow, v);
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] += sbias[l][cb + k];
+        float z[32];
+        if (!last) {   // the next product first, its operand's stores beside it
+#pragma unroll
+            for (int k = 0; k < 32; ++k) z[k] = act_apply(v[k], ACT);
+            store_bf16_32(sA, rl, cb, z);
+            fence_before();
+            fence_proxy_async();
+            __syncthreads();
+        }
+        if (pre) store_rows(pre + ((long)l * n + r0) * kTile + cb, v, turn, lane, rows);
+        store_rows(last ? Y + r0 * kTile + cb : acts + ((long)l * n + r0) * kTile + cb, last ? v : z, turn,
+                   lane, rows);
+    }
+    if (!ok && tid == 0) atomicExch(err, 1);
+    fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem);
+}
+
+struct BwdPtrs {
+    float *dW[SF_MLP_LAYERS], *db[SF_MLP_LAYERS];
+};
+
+__global__ void k_zero_db(BwdPtrs d) { d.db[blockIdx.x][threadIdx.x] = 0.f; }
+
+// A CTA takes the rows whose index modulo 256 is 4 blockIdx .. 4 blockIdx + 3, one residue for each 32
+// tile rows (32 rows 256 apart), so that db is added up as k_colsum does: one sequential FP32 sum per
+// residue, the 256 sums added by atomics.  A bias gradient is a sum that often nearly cancels and
+// Adam's first steps take its sign, so sums in another order move a bias by the learning rate.
+template <int ACT>
+__global__ void __launch_bounds__(kTrainThreads, 1) k_bwd_rows(InferW w, long n,
+        const float *__restrict__ pre, const float *__restrict__ dY, BwdPtrs d,
+        __nv_bfloat16 *__restrict__ Gb, int *err) {
+    extern __shared__ __align__(1024) unsigned char dsm[];
+    __nv_bfloat16 *sG = reinterpret_cast<__nv_bfloat16 *>(dsm), *sW = sG + kPTile;
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rb = (warp & 3) * 32, rl = rb + lane, cb = (warp >> 2) * 32;
+    float *turn = reinterpret_cast<float *>(sW + 2 * kPTile) + warp * 32 * kTurn;
+    const int res0 = blockIdx.x * 4, res = res0 + (warp & 3);
+    constexpr long kPitch = (long)kDbParts * kTile;   // from a row to the next of its residue
+    if (warp == 0) tmem_alloc(&tmem_base);
+    if (tid == 0) {
+        mbar_init(&mbar);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base, trow = ((uint32_t)rb << 16) + cb;
+    bool ok = true;
+    uint32_t ph = 0;
+    float db[SF_MLP_LAYERS] = {};   // this warp's residue, column cb + lane
+    for (long m0 = 0; m0 + res0 < n && ok; m0 += 32 * kDbParts) {
+        const long r0 = m0 + res;   // this warp's first row
+        const int rows = r0 < n ? (int)(((n - 1 - r0) / kDbParts + 1 < 32) ? (n - 1 - r0) / kDbParts + 1 : 32) : 0;
+        float v[32];
+        float4 q[8], wq[4];
+        load_weights(wq, w.W[SF_MLP_LAYERS - 1]);
+        load_rows(q, dY + r0 * kTile + cb, lane, rows, kPitch);
+        put_weights(sW, wq);
+        turn_rows(v, q, turn, lane, rows);
+#pragma unroll
+        for (int it = 0; it < SF_MLP_LAYERS; ++it) {
+            const int l = SF_MLP_LAYERS - 1 - it;
+            // v holds G_l (0 on rows past the end), also in `turn` when l = 4
+            store_bf16_32(sG, rl, cb, v);
+            fence_before();
+            fence_proxy_async();
+            __syncthreads();
+            if (l > 0 && tid == 0) {   // dA[m, in] = sum_out G[m, out] W[out, in]
+                fence_after();
+                const uint32_t a0 = smem_u32(sG), b0 = smem_u32(sW + (it & 1) * kPTile);
+                for (int s = 0; s < kTile / 16; ++s)
+                    mma_bf16_d(tmem, sdesc(a0 + s * 2 * kPLBO, kPLBO, kPSBO),
+                               sdesc(b0 + s * 2 * kPSBO, kPSBO, kPLBO), kIdesc | kMajB, s > 0);
+                mma_commit(&mbar);
+            }
+            // beside the product: the next pre-activations and weights, this layer's column sums and
+            // BF16 copy
+            if (l > 0) load_rows(q, pre + ((long)(l - 1) * n + r0) * kTile + cb, lane, rows, kPitch);
+            if (l > 1) load_weights(wq, w.W[l - 1]);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                *reinterpret_cast<float4 *>(turn + lane * kTurn + 4 * k) =
+                    make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            __syncwarp();
+            for (int r = 0; r < rows; ++r) db[l] += turn[r * kTurn + lane];
+            if (l < SF_MLP_LAYERS - 1) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int c = tid + e * kTrainThreads, r = c >> 4, k = (c & 15) * 8;
+                    const long x = m0 + res0 + (r >> 5) + (long)(r & 31) * kDbParts;
+                    if (x < n)
+                        *reinterpret_cast<uint4 *>(Gb + ((long)l * n + x) * kTile + k) =
+                            *reinterpret_cast<const uint4 *>(&sG[pcm_index(r, k)]);
+                }
+            }
+            if (l == 0) break;
+            if (l > 1) put_weights(sW + ((it + 1) & 1) * kPTile, wq);
+            float z[32];
+            turn_rows(z, q, turn, lane, rows);
+            const bool done = mbar_wait(&mbar, ph);
+            ph ^= 1;
+            fence_after();
+            if (__syncthreads_or(!done)) {
+                ok = false;
+                break;
+            }
+            tmem_ld32(tmem + trow, v);
+#pragma unroll
+            for (int k = 0; k < 32; ++k)
+                v[k] = lane < rows ? v[k] * (ACT == kActRelu ? (z[k] > 0.f ? 1.f : 0.f) : gelu_grad(z[k])) : 0.f;
+        }
+        fence_before();
+        __syncthreads();   // sG has been copied out before the next chunk's first layer
+    }
+    if (ok && res < n) {
+#pragma unroll
+        for (int l = 0; l < SF_MLP_LAYERS; ++l) atomicAdd(&d.db[l][cb + lane], db[l]);
+    }
+    if (!ok && tid == 0) atomicExch(err, 1);
+    fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem);
+}
+
+// dW_l[:, c0 .. c0+31] = G_l^T X_l, all rows in order into one accumulator (LAST: the last layer, whose
+// G is dY in FP32).  The next 256 rows' loads are in registers while the current ones are
+// multiplied (two staging buffers, each freed by the commit of its products).
+template <bool LAST>
+__device__ __forceinline__ void bwd_dw(long n, const float *__restrict__ Xl, const float *__restrict__ dY,
+                                       const __nv_bfloat16 *__restrict__ Gl, int c0,
+                                       float *__restrict__ dW, int *err) {
+    extern __shared__ __align__(1024) unsigned char dsm[];
+    __shared__ __align__(8) uint64_t mbar[2];
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) tmem_alloc(&tmem_base);
+    if (tid == 0) {
+        mbar_init(&mbar[0]);
+        mbar_init(&mbar[1]);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_base;
+    constexpr uint32_t idesc = ((kIdesc & ~(0x3Fu << 17)) | ((uint32_t)(kDwCols >> 3) << 17)) | kMajA | kMajB;
+    const int ntiles = (int)((n + kDwRows - 1) / kDwRows);
+    // the loads carry no branch and no conversion (which would wait for each load in turn): rows past
+    // the end load the last row and are zeroed when they are staged
+    constexpr int kG = (LAST ? 8 : 4) * (kDwRows / kTile), kX = 2 * (kDwRows / kTile);
+    float4 g[kG], x[kX];
+    auto load = [&](int t) {
+#pragma unroll
+        for (int q = 0; q < kG; ++q) {   // G: 4 columns a thread in FP32, 8 in BF16
+            const int e = tid + q * kTrainThreads;
+            const long ra = (long)t * kDwRows + (LAST ? e >> 5 : e >> 4), r = ra < n ? ra : n - 1;
+            g[q] = LAST ? ld_now(dY + r * kTile + (e & 31) * 4) : ld_now(Gl + r * kTile + (e & 15) * 8);
+        }
+#pragma unroll
+        for (int q = 0; q < kX; ++q) {   // X: 4 columns a thread
+            const int e = tid + q * kTrainThreads;
+            const long ra = (long)t * kDwRows + (e >> 3), r = ra < n ? ra : n - 1;
+            x[q] = ld_now(Xl + r * kTile + c0 + (e & 7) * 4);
+        }
+    };
+    bool ok = true;
+    load(0);
+    for (int t = 0; t < ntiles; ++t) {
+        const int b = t & 1;
+        __nv_bfloat16 *sG = reinterpret_cast<__nv_bfloat16 *>(dsm + b * kDwStage), *sX = sG + (kDwRows / 8) * (kPSBO / 2);
+        const long left = n - (long)t * kDwRows;   // rows of this tile
+        if (t >= 2) {
+            const bool done = mbar_wait(&mbar[b], ((t >> 1) - 1) & 1);
+            if (__syncthreads_or(!done)) {
+                ok = false;
+                break;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kG; ++q) {
+            const int e = tid + q * kTrainThreads, r = LAST ? e >> 5 : e >> 4;
+            const float4 v = r < left ? g[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (LAST)
+                *reinterpret_cast<uint2 *>(&sG[pcm_index(r, (e & 31) * 4)]) =
+                    make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+            else
+                *reinterpret_cast<float4 *>(&sG[pcm_index(r, (e & 15) * 8)]) = v;
+        }
+#pragma unroll
+        for (int q = 0; q < kX; ++q) {
+            const int e = tid + q * kTrainThreads, r = e >> 3;
+            const float4 v = r < left ? x[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<uint2 *>(&sX[pcm_index(r, (e & 7) * 4, kDwCols / 8)]) =
+                make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+        }
+        fence_proxy_async();
+        __syncthreads();
+        if (tid == 0) {   // D[out, in] += sum_m G[m, out] X[m, in], 16 rows m a step
+            const uint32_t a0 = smem_u32(sG), b0 = smem_u32(sX);
+            for (int s = 0; s < kDwRows / 16 && s * 16 < left; ++s)
+                mma_bf16_d(tmem, sdesc(a0 + s * 2 * kPSBO, kPSBO, kPLBO),
+                           sdesc(b0 + s * 2 * kDwKB, kDwKB, kPLBO), idesc, (t > 0 || s > 0) ? 1u : 0u);
+            mma_commit(&mbar[b]);
+        }
+        // after the products are issued: before the fence they would be waited for there (123 us
+        // against 93 with 128 rows a stage)
+        if (t + 1 < ntiles) load(t + 1);
+    }
+    if (ok) {   // the last commit covers every product before it
+        const bool done = mbar_wait(&mbar[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1);
+        if (__syncthreads_or(!done)) ok = false;
+    }
+    fence_after();
+    if (ok && warp < 4) {
+        float v[32];
+        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), v);
+        store_rows(dW + warp * 32 * kTile + c0, v, reinterpret_cast<float *>(dsm) + warp * 32 * kTurn, lane, 32);
+    }
+    if (!ok && tid == 0) atomicExch(err, 1);
+    fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem);
+}
+
+// blockIdx = (32 input columns, layer)
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    k_bwd_dw(long n, const float *__restrict__ X, const float *__restrict__ acts,
+             const float *__restrict__ dY, const __nv_bfloat16 *__restrict__ Gb, BwdPtrs d, int *err) {
+    const int c0 = blockIdx.x * kDwCols, l = blockIdx.y;
+    const float *Xl = l == 0 ? X : acts + (long)(l - 1) * n * kTile;
+    if (l == SF_MLP_LAYERS - 1) bwd_dw<true>(n, Xl, dY, nullptr, c0, d.dW[l], err);
+    else bwd_dw<false>(n, Xl, nullptr, Gb + (long)l * n * kTile, c0, d.dW[l], err);
 }
 
 }  // namespace mlp
@@ -855,6 +1288,50 @@ int mcuda(cudaError_t e, const char *where) {
 }
 inline cudaStream_t S(sf_stream s) { return reinterpret_cast<cudaStream_t>(s); }
 inline unsigned nblk(long n, int b) { return (unsigned)((n + b - 1) / b); }
+
+sf::mlp::InferW infer_w(const sf_mlp_params *w) {
+    sf::mlp::InferW iw;
+    for (int l = 0; l < SF_MLP_LAYERS; ++l) {
+        iw.W[l] = static_cast<const __nv_bfloat16 *>(w->W[l]);
+        iw.b[l] = w->b[l];
+    }
+    return iw;
+}
+
+// The fused training passes read and write 16 bytes at a time: every buffer and the weights of
+// layers l0.. on 16-byte boundaries; otherwise the passes run layer by layer (k_gemm).
+bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+bool fused_ok(const sf_mlp_params *w, int l0, std::initializer_list<const void *> bufs) {
+    for (const void *p : bufs)
+        if (!aligned16(p)) return false;
+    for (int l = l0; l < SF_MLP_LAYERS; ++l)
+        if (!w->W[l] || !aligned16(w->W[l])) return false;
+    return true;
+}
+bool grads_ok(float *const *dW, float *const *db) {
+    for (int l = 0; l < SF_MLP_LAYERS; ++l)
+        if (!dW[l] || !db[l] || !aligned16(dW[l])) return false;
+    return true;
+}
+
+// The raised shared-memory limits are per-device function attributes: set once on each device.
+int train_attrs() {
+    static bool done[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return mcuda(e, "cudaGetDevice");
+    if (dev >= 0 && dev < 64 && done[dev]) return SF_OK;
+    const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    using namespace sf::mlp;
+    for (auto k : {k_fwd<kActGelu>, k_fwd<kActRelu>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, (int)kRowsSmem);
+    for (auto k : {k_bwd_rows<kActGelu>, k_bwd_rows<kActRelu>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, (int)kRowsSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_bwd_dw, at, (int)kDwSmem);
+    if (e != cudaSuccess) return mcuda(e, "cudaFuncSetAttribute");
+    if (dev >= 0 && dev < 64) done[dev] = true;
+    return SF_OK;
+}
 }  // namespace
 
 using sf::mlp::Mat;
@@ -892,6 +1369,15 @@ int sf_mlp_gemm(int n_rows, int K, const void *A, int a_bf16, long a_rs, long a_
 int sf_mlp_forward(const sf_mlp_params *w, int n, const float *X, float *Y, float *acts,
                    float *pre, int *err, sf_stream s) {
     if (!w || !X || !Y || n <= 0) return mfail(SF_EINVAL, "bad argument");
+    if (acts && err && fused_ok(w, 0, {X, Y, acts, pre})) {
+        int rc = train_attrs();
+        if (rc) return rc;
+        auto k = w->act == SF_MLP_RELU ? sf::mlp::k_fwd<sf::mlp::kActRelu> : sf::mlp::k_fwd<sf::mlp::kActGelu>;
+        k<<<nblk(n, kTile), sf::mlp::kTrainThreads, sf::mlp::kRowsSmem, S(s)>>>(infer_w(w), n, X, Y, acts,
+                                                                               pre, err);
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_forward");
+    }
     const long ld = kTile;
     const float *in = X;
     for (int l = 0; l < SF_MLP_LAYERS; ++l) {
@@ -913,6 +1399,25 @@ int sf_mlp_backward(const sf_mlp_params *w, int n, const float *X, const float *
                     float *work, int *err, sf_stream s) {
     if (!w || !X || !acts || !pre || !dY || !dW || !db || !work || n <= 0 || n % 16)
         return mfail(SF_EINVAL, "bad argument (n must be a multiple of 16)");
+    if (err && fused_ok(w, 1, {X, acts, pre, dY, work}) && grads_ok(dW, db)) {
+        int rc = train_attrs();
+        if (rc) return rc;
+        sf::mlp::BwdPtrs d;
+        for (int l = 0; l < SF_MLP_LAYERS; ++l) {
+            d.dW[l] = dW[l];
+            d.db[l] = db[l];
+        }
+        auto *Gb = reinterpret_cast<__nv_bfloat16 *>(work);   // 4 layers x n x 128 BF16: all of it
+        sf::mlp::k_zero_db<<<SF_MLP_LAYERS, kTile, 0, S(s)>>>(d);
+        auto k = w->act == SF_MLP_RELU ? sf::mlp::k_bwd_rows<sf::mlp::kActRelu>
+                                       : sf::mlp::k_bwd_rows<sf::mlp::kActGelu>;
+        k<<<sf::mlp::kDbParts / 4, sf::mlp::kTrainThreads, sf::mlp::kRowsSmem, S(s)>>>(infer_w(w), n, pre, dY, d,
+                                                                                      Gb, err);
+        sf::mlp::k_bwd_dw<<<dim3(kTile / sf::mlp::kDwCols, SF_MLP_LAYERS),
+                            sf::mlp::kTrainThreads, sf::mlp::kDwSmem, S(s)>>>(n, X, acts, dY, Gb, d, err);
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_backward");
+    }
     const long ld = kTile;
     float *G = work, *dA = work + (long)n * ld;
     const float *g_in = dY;   // gradient w.r.t. the current layer's output
@@ -933,7 +1438,7 @@ int sf_mlp_backward(const sf_mlp_params *w, int n, const float *X, const float *
         if (rc) return rc;
         const cudaError_t ez = cudaMemsetAsync(db[l], 0, sizeof(float) * kTile, S(s));
         if (ez != cudaSuccess) return mcuda(ez, "sf_mlp_backward: clearing db");
-        sf::mlp::k_colsum<<<256, kTile, 0, S(s)>>>(n, G, db[l]);
+        sf::mlp::k_colsum<<<sf::mlp::kDbParts, kTile, 0, S(s)>>>(n, G, db[l]);
         if (l > 0) {   // dA[m, in] = sum_out G[m, out] W[out, in]
             rc = sf_mlp_gemm(n, kTile, G, 0, ld, 1, w->W[l], 1, 1, ld, nullptr, 0, dA, ld, nullptr, 0,
                              err, s);
