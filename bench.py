@@ -127,10 +127,10 @@ def launches_per_step(m, mixing):
     from sailfish_b200._lib import lib
     mix = {"none": 0, "gls": 1, "mlp": 3}[mixing]
     if getattr(m, "semantics", "reference") == "roms":
-        # maxflux/omega, rhs3d, stress3d, set_depth, step3d_uv, lateral BC, walls; per substep
-        # the predictor's and the corrector's free surface and momentum (the last substep:
-        # the predictor's averages only)
-        return 7 + 4 * m.nfast + 1 + mix
+        # maxflux/omega, rhs3d, stress3d, set_depth, step3d_uv, lateral BC, walls, and the loop's
+        # launches as the model counts them (four per substep and one for the averages of the
+        # last substep, for a model that does not)
+        return 7 + getattr(m, "loop_launches", 4 * m.nfast + 1) + mix
     fused = bool(lib.sf_ctx_fused_available(m.ctx.ptr))
     sub = 4 if fused else 7
     return 4 + sub * (m.nfast + 1) + 2 + mix

@@ -240,6 +240,10 @@ int sf_roms_barotropic_loop(sf_ctx *ctx, sf_state2d *s, double *DU_avg2, double 
  * main2d's step (nonlinear/main2d.py:9-88); first selects forward/backward Euler. */
 int sf_roms_step2d(sf_ctx *ctx, sf_state2d *s, const void *sustr, const void *svstr,
                    double rdrag2, double dtfast, int first, sf_stream stream);
+/* nsteps such steps in one call (first applies to the first of them), with the results and the final
+ * slots of as many sf_roms_step2d calls. */
+int sf_roms_steps2d(sf_ctx *ctx, sf_state2d *s, const void *sustr, const void *svstr,
+                    double rdrag2, double dtfast, int nsteps, int first, sf_stream stream);
 /* Surface and bottom stress on the 3D momentum right-hand side (ROMS's ru includes them):
  * ru[N-1] += sustr om_u on_u and ru[0] -= rdrag2 ub sqrt(ub^2 + v_u^2) om_u on_u at the interior
  * U faces (ub, v_u from the bottom level of u, v), rv likewise. */

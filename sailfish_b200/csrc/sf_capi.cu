@@ -195,6 +195,8 @@ void free_ctx(sf_ctx *c) {
     cudaFree(c->bm_128);
     for (int2 *b : c->bm_tile) cudaFree(b);
     cudaFree(c->bm_pipe);
+    cudaFree(c->bm_roms);
+    cudaFree(c->bm_sub);
     delete[] c->h_off2;
     delete[] c->h_off3;
     delete[] c->h_offN;
@@ -310,6 +312,14 @@ int build_pred_maps(sf_ctx *c, const ProgHost &Z, const ProgHost &U, const ProgH
         c->pred_ok = 1;
     }
     return rc;
+}
+
+// Rows a warp of the ROMS-form barotropic phases walks: more rows load the shared rows less often,
+// fewer give more warps and a shorter chain.  52 substeps of two launches in FP32, rows 1, 2, 4, 8, 16:
+// 130 x 66 (FP64) 0.38, 0.50, 0.71, 1.16, 2.05 ms; 514 x 258 0.58, 0.60, 0.78, 1.28, 1.73;
+// 1026 x 514 1.82, 1.40, 1.26, 1.33, 2.38; 2050 x 1026 9.57, 7.11, 6.05, 5.57, 5.66.
+int roms_rows_for(long points) {
+    return points >= (1L << 20) ? 8 : points >= (1L << 18) ? 4 : points >= (1L << 16) ? 2 : 1;
 }
 
 template <typename R>
@@ -453,7 +463,8 @@ int sf_ctx_create_ensemble(const sf_grid_desc *d, int n, sf_ctx **out) {
         rc = c->prec == SF_FP64 ? upload_members<double>(c, d, n, off2, off3, offN, voff)
                                 : upload_members<float>(c, d, n, off2, off3, offN, voff);
     if (rc == SF_OK) {   // block maps
-        std::vector<int2> pt, b128, pipe, tile[sf::kRhsTiles];
+        c->roms_rows = roms_rows_for(t2);
+        std::vector<int2> pt, b128, pipe, roms, sub, tile[sf::kRhsTiles];
         for (int m = 0; m < n; ++m) {
             const int I = d[m].L + 1, J = d[m].M + 1;
             const long s2 = (long)I * J;
@@ -465,6 +476,12 @@ int sf_ctx_create_ensemble(const sf_grid_desc *d, int n, sf_ctx **out) {
                 for (int b = 0; b < ntx * nty; ++b) tile[v].push_back({m, b});
             }
             for (long b = 0; b < (s2 + sf::kPipeTile - 1) / sf::kPipeTile; ++b) pipe.push_back({m, (int)b});
+            const int br = c->roms_rows * sf::kRomsWarps;
+            const int nb = (I + sf::kRomsCols - 1) / sf::kRomsCols * ((J + br - 1) / br);
+            for (int b = 0; b < nb; ++b) roms.push_back({m, b});
+            const int bs = sf::kSubRows - 3;
+            const int nsub = (I + sf::kSubCols - 1) / sf::kSubCols * ((J + bs - 1) / bs);
+            for (int b = 0; b < nsub; ++b) sub.push_back({m, b});
         }
         c->nbm_pt = (int)pt.size();
         c->nbm_128 = (int)b128.size();
@@ -472,6 +489,10 @@ int sf_ctx_create_ensemble(const sf_grid_desc *d, int n, sf_ctx **out) {
         rc = upload(&c->bm_pt, pt.data(), pt.size(), "block map");
         if (rc == SF_OK) rc = upload(&c->bm_128, b128.data(), b128.size(), "block map");
         if (rc == SF_OK) rc = upload(&c->bm_pipe, pipe.data(), pipe.size(), "block map");
+        c->nbm_roms = (int)roms.size();
+        if (rc == SF_OK) rc = upload(&c->bm_roms, roms.data(), roms.size(), "block map");
+        c->nbm_sub = (int)sub.size();
+        if (rc == SF_OK) rc = upload(&c->bm_sub, sub.data(), sub.size(), "block map");
         for (int v = 0; v < sf::kRhsTiles && rc == SF_OK; ++v) {
             c->nbm_tile[v] = (int)tile[v].size();
             rc = upload(&c->bm_tile[v], tile[v].data(), tile[v].size(), "block map");
@@ -531,6 +552,7 @@ int sf_ctx_create(const sf_grid_desc *d, sf_ctx **out) {
     c->I = d->L + 1;
     c->J = d->M + 1;
     c->s2 = (long)c->I * c->J;
+    c->roms_rows = roms_rows_for(c->s2);
     c->hc = d->hc;
     c->Vtransform = d->Vtransform;
     // horizontalAdvection is launched with (grsz*GPUMUL, bksz//GPUMUL) = 512*(s2/512 + 1)
@@ -1019,32 +1041,23 @@ int sf_barotropic_loop(sf_ctx *c, sf_state2d *st, int nsub, const double *weight
 }  // extern "C"
 
 namespace {
-// One phase (0 predictor, 1 corrector) of the ROMS-form substep on the slots of st:
-// [0] = n-1, [1] = n, [2] = the predicted n+1*.
+// One phase (0 predictor, 1 corrector, 2 accumulation only, 3 a whole substep) of the ROMS-form
+// substep on the slots of st: [0] = n-1, [1] = n, [2] = the predicted n+1* (3: the new level).
 template <typename R>
 cudaError_t roms_phase(const sf_ctx *c, const sf_state2d *st, double *DU2, double *DV2,
                        const void *sustr, const void *svstr, double rdrag2, double dtfast,
-                       int phase, int first, int acc, double c1, double c2, int step,
+                       int phase, int first, int acc, double c1, double c2, double c2c,
                        cudaStream_t s) {
     sf::RomsArgs<R> a;
-    a.zb = (const R *)st->zeta[0];
-    a.zn = (const R *)st->zeta[1];
-    a.zp = (const R *)st->zeta[2];
-    a.ub = (const R *)st->ubar[0];
-    a.un = (const R *)st->ubar[1];
-    a.up = (const R *)st->ubar[2];
-    a.vb = (const R *)st->vbar[0];
-    a.vn = (const R *)st->vbar[1];
-    a.vp = (const R *)st->vbar[2];
-    const int out = phase == 0 ? 2 : 0;
+    const int out = phase == 1 ? 0 : 2;
     a.zout = (R *)st->zeta[out];
     a.uout = (R *)st->ubar[out];
     a.vout = (R *)st->vbar[out];
-    const int kstp = phase == 0 ? (first ? 1 : 0) : 1;
+    const int kstp = phase == 1 || first ? 1 : 0;
     a.zkstp = (const R *)st->zeta[kstp];
     a.ukstp = (const R *)st->ubar[kstp];
     a.vkstp = (const R *)st->vbar[kstp];
-    const int krhs = phase == 0 ? 1 : 2;
+    const int krhs = phase == 1 ? 2 : 1;
     a.zrhs = (const R *)st->zeta[krhs];
     a.urhs = (const R *)st->ubar[krhs];
     a.vrhs = (const R *)st->vbar[krhs];
@@ -1065,12 +1078,34 @@ cudaError_t roms_phase(const sf_ctx *c, const sf_state2d *st, double *DU2, doubl
     a.dtfast = dtfast;
     a.c1 = c1;
     a.c2 = c2;
+    a.c2c = c2c;
     a.phase = phase;
     a.first = first;
     a.acc = acc;
-    a.step = step;
     return sf::Ops<R>::roms_phase(c, a, s);
 }
+
+// After a fused substep, whose n+1 is in the scratch slot of zeta, ubar, vbar: these rotate, the
+// tendencies swap.
+void roms_rotate(sf_state2d *st) {
+    for (void **a : {st->zeta, st->ubar, st->vbar}) {
+        void *t = a[0];
+        a[0] = a[1];
+        a[1] = a[2];
+        a[2] = t;
+    }
+    for (void **a : {st->rzeta, st->rubar, st->rvbar}) {
+        void *t = a[0];
+        a[0] = a[1];
+        a[1] = t;
+    }
+}
+
+// Leapfrog substeps to run fused of `left` to come: groups of six, after which every slot is back
+// in its place (the levels rotate with period 3, the tendencies with 2), and at least one not fused,
+// so that the scratch slot ends with the predicted level: the caller's slots end as from substeps
+// of two launches each.
+int roms_fused(int left) { return left > 0 ? (left - 1) / 6 * 6 : 0; }
 
 void roms_swap(sf_state2d *st) {   // n+1 (written over n-1) becomes n, n becomes n-1
     void **arrs[6] = {st->zeta, st->ubar, st->vbar, st->rzeta, st->rubar, st->rvbar};
@@ -1104,6 +1139,7 @@ int sf_roms_barotropic_loop(sf_ctx *c, sf_state2d *st, double *DU_avg2, double *
     if (!DU_avg2 || !DV_avg2 || !st->Zt_avg1 || !st->DU_avg1 || !st->DV_avg1 || !W1 || !W2)
         return fail(SF_EINVAL, "null accumulator or weights");
     if (nfast < 1 || nfast > 254) return fail(SF_EINVAL, "nfast must be in [1, 254]");
+    const int nfused = roms_fused(nfast - 1);
     for (int iif = 1; iif <= nfast + 1; ++iif) {
         // fast-time averages (step2d_LF_AM3.h.py:778-846), ROMS-indexed weights
         const int acc = iif == 1 ? 2 : 1;
@@ -1112,37 +1148,48 @@ int sf_roms_barotropic_loop(sf_ctx *c, sf_state2d *st, double *DU_avg2, double *
                                     : (8.0 / 12.0) * W2[iif] - (1.0 / 12.0) * W2[iif + 1];
         const double cc2 = iif == 1 ? W2[1] : (5.0 / 12.0) * W2[iif];
         const int step = iif <= nfast, first = iif == 1;
-        cudaError_t e = c->prec == SF_FP64
-            ? roms_phase<double>(c, st, DU_avg2, DV_avg2, sustr, svstr, rdrag2, dtfast, 0, first,
-                                 acc, pc1, pc2, step, S(s))
-            : roms_phase<float>(c, st, DU_avg2, DV_avg2, sustr, svstr, rdrag2, dtfast, 0, first,
-                                acc, pc1, pc2, step, S(s));
-        if (e == cudaSuccess && step)
+        cudaError_t e = cudaSuccess;
+        const bool fused = step && !first && iif - 2 < nfused;
+        const int ph0 = fused ? 3 : (step ? 0 : 2), ph1 = fused ? 3 : (step ? 1 : 2);
+        for (int ph = ph0; ph <= ph1 && e == cudaSuccess; ++ph)
             e = c->prec == SF_FP64
-                ? roms_phase<double>(c, st, DU_avg2, DV_avg2, sustr, svstr, rdrag2, dtfast, 1,
-                                     first, 1, 0.0, cc2, 1, S(s))
-                : roms_phase<float>(c, st, DU_avg2, DV_avg2, sustr, svstr, rdrag2, dtfast, 1,
-                                    first, 1, 0.0, cc2, 1, S(s));
+                ? roms_phase<double>(c, st, DU_avg2, DV_avg2, sustr, svstr, rdrag2, dtfast, ph,
+                                     first, acc, pc1, pc2, cc2, S(s))
+                : roms_phase<float>(c, st, DU_avg2, DV_avg2, sustr, svstr, rdrag2, dtfast, ph,
+                                    first, acc, pc1, pc2, cc2, S(s));
         if (e != cudaSuccess) return cuda_fail(e, "sf_roms_barotropic_loop");
-        if (step) roms_swap(st);
+        if (fused) roms_rotate(st);
+        else if (step) roms_swap(st);
+    }
+    return SF_OK;
+}
+
+int sf_roms_steps2d(sf_ctx *c, sf_state2d *st, const void *sustr, const void *svstr,
+                    double rdrag2, double dtfast, int nsteps, int first, sf_stream s) {
+    int rc = roms_check(c, st, sustr, svstr);
+    if (rc) return rc;
+    if (nsteps < 0) return fail(SF_EINVAL, "nsteps must not be negative");
+    const int f0 = first ? 1 : 0, nfused = roms_fused(nsteps - f0);
+    for (int k = 0; k < nsteps; ++k) {
+        const bool fused = k >= f0 && k - f0 < nfused;
+        const int f = k < f0 ? 1 : 0;
+        cudaError_t e = cudaSuccess;
+        for (int ph = fused ? 3 : 0; ph <= (fused ? 3 : 1) && e == cudaSuccess; ++ph)
+            e = c->prec == SF_FP64
+                ? roms_phase<double>(c, st, nullptr, nullptr, sustr, svstr, rdrag2, dtfast, ph, f, 0,
+                                     0.0, 0.0, 0.0, S(s))
+                : roms_phase<float>(c, st, nullptr, nullptr, sustr, svstr, rdrag2, dtfast, ph, f, 0,
+                                    0.0, 0.0, 0.0, S(s));
+        if (e != cudaSuccess) return cuda_fail(e, "sf_roms_steps2d");
+        if (fused) roms_rotate(st);
+        else roms_swap(st);
     }
     return SF_OK;
 }
 
 int sf_roms_step2d(sf_ctx *c, sf_state2d *st, const void *sustr, const void *svstr,
                    double rdrag2, double dtfast, int first, sf_stream s) {
-    int rc = roms_check(c, st, sustr, svstr);
-    if (rc) return rc;
-    cudaError_t e = cudaSuccess;
-    for (int phase = 0; phase < 2 && e == cudaSuccess; ++phase)
-        e = c->prec == SF_FP64
-            ? roms_phase<double>(c, st, nullptr, nullptr, sustr, svstr, rdrag2, dtfast, phase,
-                                 first ? 1 : 0, 0, 0.0, 0.0, 1, S(s))
-            : roms_phase<float>(c, st, nullptr, nullptr, sustr, svstr, rdrag2, dtfast, phase,
-                                first ? 1 : 0, 0, 0.0, 0.0, 1, S(s));
-    if (e != cudaSuccess) return cuda_fail(e, "sf_roms_step2d");
-    roms_swap(st);
-    return SF_OK;
+    return sf_roms_steps2d(c, st, sustr, svstr, rdrag2, dtfast, 1, first, s);
 }
 
 static double ab3_cff(int iic, int ntfirst) {   // step3D_uv.kernels.cpp:663-666

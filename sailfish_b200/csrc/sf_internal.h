@@ -170,6 +170,11 @@ struct sf_ctx {
     int2 *bm_tile[sf::kRhsTiles] = {};   // tiles of the tiled 3D right-hand side, per variant
     int nbm_tile[sf::kRhsTiles] = {};
     int rhs_tile = 0;            // variant of the tiled 3D right-hand side (sf_ctx_set_tile)
+    int2 *bm_roms = nullptr;     // strips of the ROMS-form barotropic phases
+    int nbm_roms = 0;
+    int2 *bm_sub = nullptr;      // tiles of the fused substep
+    int nbm_sub = 0;
+    int roms_rows = 8;           // rows a warp of those phases walks (roms_rows_for)
     int2 *bm_pipe = nullptr;     // 64-point tiles of the pipelined column solve
     int nbm_pipe = 0;
     long tot2 = 0, tot3 = 0, totN = 0;   // pool sizes
@@ -216,24 +221,26 @@ constexpr int kRomsMaxN = 64;
 // Arguments of one phase of the ROMS-form barotropic substep (kernels in sf_roms.cuh).
 template <typename R>
 struct RomsArgs {
-    const R *zb, *zn, *zp;          // zeta at n-1, n and the predicted n+1*
-    const R *ub, *un, *up;
-    const R *vb, *vn, *vp;
+    const R *zrhs, *urhs, *vrhs;    // the level of the fluxes and the right-hand side (krhs)
+    const R *zkstp, *ukstp, *vkstp; // the old level (kstp; level n in the corrector)
     R *zout, *uout, *vout;          // the phase's output slots (p in the predictor, b in the corrector)
-    const R *zkstp, *ukstp, *vkstp; // the momentum step's old level (kstp)
-    const R *zrhs, *urhs, *vrhs;    // the level the right-hand side is evaluated at (krhs)
     R *rz_n, *ru_n, *rv_n;          // tendencies of level n (written by the predictor)
     const R *rz_b, *ru_b, *rv_b;    // tendencies of level n-1
     const R *sustr, *svstr;         // kinematic surface stress at U / V faces (m2/s2)
     double *Zt, *DU1, *DV1, *DU2, *DV2;
     double rdrag2, dtfast;
-    double c1, c2;                  // accumulation weights of this phase
-    int phase;                      // 0 predictor, 1 corrector
+    double c1, c2, c2c;             // accumulation weights: the predictor's, the corrector's
+    int phase;                      // 0 predictor, 1 corrector, 2 the last substep's accumulation,
+                                    // 3 a whole substep (fused)
     int first;                      // first substep of a loop: forward / backward Euler
-    int acc;                        // 0 none, 1 accumulate, 2 reset (predictor of substep 1)
-    int step;                       // 0: the predictor only accumulates (substep nfast+1)
+    int acc;                        // 0 none, 1 accumulate, 2 reset (substep 1)
 };
 
+// Strips of the barotropic phases: columns a warp writes, warps (runs of rows) per block.
+constexpr int kRomsCols = 29, kRomsWarps = 4;
+// Tiles of the fused substep: columns of its own, staged rows (3 more than its own).  Rows measured
+// at 2050 x 1026 in FP32: 8, 12, 16, 24 staged rows 4.82, 4.35, 5.07, 6.61 ms a loop.
+constexpr int kSubCols = 27, kSubRows = 12;
 
 // Launchers, one explicit instantiation per precision (FP64 in a translation unit built
 // without FMA contraction, so that it reproduces the reference's IEEE evaluation).

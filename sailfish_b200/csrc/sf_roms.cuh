@@ -12,161 +12,489 @@
 // ubar(p) on the west face of rho p, vbar(p) on its south face; interior rho i = 1..I-2,
 // j = 1..J-2; interior U faces i = 2..I-2 (walls i = 1, I-1), V faces j = 2..J-2.
 //
-// A substep is four launches: the predictor's free surface (k_roms_zeta, phase 0), its
-// momentum (k_roms_mom, phase 0), the corrector's free surface (phase 1) and momentum
-// (phase 1).  Time levels: slots b (n-1), n and p (the predicted n+1*); the corrector writes
-// n+1 into b and the host swaps b and n.  Every expression keeps the operand order of the
-// oracle's restatement (oracle/roms_oracle.py), so the FP64 build (no FMA contraction)
-// reproduces it bit for bit; the fast-time averages are FP64 in both precisions.
+// A substep is two launches: the predictor (free surface, then momentum) and the corrector, each by
+// warps that walk up the rows of a strip of columns (roms_phase_rows).  Time levels: slots b
+// (n-1), n and p (the predicted n+1*); the corrector writes n+1 into b and the host swaps b and
+// n.  Every expression keeps the operand order of the oracle's restatement
+// (oracle/roms_oracle.py), so the FP64 build (no FMA contraction) reproduces it bit for bit; the
+// fast-time averages are FP64 in both precisions.
 #pragma once
 
 namespace sf {
 
 
-// DUon at the U face p (0 on column 0) and DVom at the V face p (0 on row 0), from zeta, ubar, vbar
-template <typename R>
-__device__ __forceinline__ R roms_du(const Geo<R> &g, const R *z, const R *u, long p, int i) {
-    if (i < 1) return R(0);
-    const R Dp = z[p] + g.h[p], Dw = z[p - 1] + g.h[p - 1];
-    return (u[p] * (R(0.5) * (Dp + Dw))) * g.on_u[p];
-}
-template <typename R>
-__device__ __forceinline__ R roms_dv(const Geo<R> &g, const R *z, const R *v, long p, int j) {
-    if (j < 1) return R(0);
-    const R Dp = z[p] + g.h[p], Ds = z[p - g.I] + g.h[p - g.I];
-    return (v[p] * (R(0.5) * (Dp + Ds))) * g.om_v[p];
-}
-// rhs_zeta at interior rho q: (DUon_q - DUon_q+1) + (DVom_q - DVom_q+I)
-template <typename R>
-__device__ __forceinline__ R roms_rz(const Geo<R> &g, const R *z, const R *u, const R *v, long q,
-                                     int i, int j) {
-    return (roms_du(g, z, u, q, i) - roms_du(g, z, u, q + 1, i + 1)) +
-           (roms_dv(g, z, v, q, j) - roms_dv(g, z, v, q + g.I, j + 1));
+// The barotropic phases are launched with programmatic dependent launch (as the reference form's
+// loop): a kernel's blocks become resident while its predecessor runs and wait for its completion on
+// the device.  They let their own successor in only after that wait: at most one launch waits in
+// the SMs, so that the running one's blocks spread over all of them (with the order the other way
+// round blocks of several waiting launches take the places: 258 x 130 nodes in FP32, 6.9 us a substep
+// against 3.4).
+__device__ __forceinline__ void pdl_wait_then_launch() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Free surface of a phase at rho p.  Ring nodes take the value of the nearest interior node
-// (zero gradient at closed walls), computed here from the inputs.
+// The barotropic substep's products and sums, with the FP32 form's contractions written out: a product
+// either rounds by itself (rmul) or goes into one fused multiply-add (rfma), so that every form of
+// the substep (two launches, fused; single grid, ensemble) gives the same bits whatever the compiler
+// would fuse in it.  The FP64 form rounds every product and sum, as the oracle does.
 template <typename R>
-__device__ __forceinline__ void roms_zeta_at(const Geo<R> &g, const RomsArgs<R> &a, const long p) {
-    if (p >= g.s2) return;
-    const int j = fdiv((int)p, g.dI), i = (int)p - j * g.I;
-    const long I = g.I;
-    if (a.acc) {   // the fast-time averages at rho p, its west U face and its south V face
-        const R *z = a.phase == 0 ? a.zn : a.zp;
-        const R *u = a.phase == 0 ? a.un : a.up;
-        const R *v = a.phase == 0 ? a.vn : a.vp;
-        const double du = (double)roms_du(g, z, u, p, i), dv = (double)roms_dv(g, z, v, p, j);
-        if (a.phase == 0) {
-            if (a.acc == 2) {
-                a.Zt[p] = 0.0;
-                a.DU1[p] = 0.0;
-                a.DV1[p] = 0.0;
-                a.DU2[p] = a.c2 * du;
-                a.DV2[p] = a.c2 * dv;
-            } else {
-                a.Zt[p] = a.Zt[p] + a.c1 * (double)z[p];
-                a.DU1[p] = a.DU1[p] + a.c1 * du;
-                a.DV1[p] = a.DV1[p] + a.c1 * dv;
-                a.DU2[p] = a.DU2[p] + a.c2 * du;
-                a.DV2[p] = a.DV2[p] + a.c2 * dv;
-            }
-        } else {
-            a.DU2[p] = a.DU2[p] + a.c2 * du;
-            a.DV2[p] = a.DV2[p] + a.c2 * dv;
+__device__ __forceinline__ R rmul(R a, R b) {
+    if constexpr (sizeof(R) == 4) return __fmul_rn(a, b);
+    else return a * b;
+}
+template <typename R>
+__device__ __forceinline__ R rfma(R a, R b, R c) {
+    if constexpr (sizeof(R) == 4) return __fmaf_rn(a, b, c);
+    else return a * b + c;
+}
+// an FP64 average plus a weighted term
+template <typename R>
+__device__ __forceinline__ double rsum(double s, double c, double x) {
+    if constexpr (sizeof(R) == 4) return __fma_rn(c, x, s);
+    else return s + c * x;
+}
+template <typename R>
+__device__ __forceinline__ R roms_am3(R r, R rn, R rb) {
+    return rfma(-R(1.0 / 12.0), rb, rfma(R(5.0 / 12.0), r, rmul(R(8.0 / 12.0), rn)));
+}
+// The momentum right-hand side at a face: gm, hm the pressure-gradient surface and depth on its minus
+// side, gp, h on its plus side; u the velocity there, o4 the four-point average of the other
+// component; cor the sum of the two Coriolis fluxes; area 4 / ((pm + pm)(pn + pn)).
+template <typename R, bool V>
+__device__ __forceinline__ R roms_rhs(R met, R gm, R gp, R hm, R h, R cor, R u, R o4, R rdrag2, R str, R area) {
+    const R cffg = R(0.5 * 10.0);   // 0.5 g, g = 10 (mod_constants.py:26)
+    const R in = rfma(hm + h, gm - gp, rfma(gm, gm, -rmul(gp, gp)));
+    const R pa = rmul(cffg, met);
+    const R pc = V ? rmul(pa, in) + rmul(R(-0.5), cor) : rfma(pa, in, rmul(R(0.5), cor));
+    const R tau = rfma(-rmul(rdrag2, u), sqrt(rfma(u, u, rmul(o4, o4))), str);
+    return rfma(tau, area, pc);
+}
+// A face's new velocity: (u Ds + pmn2 cdt f) / Dn.
+template <typename R>
+__device__ __forceinline__ R roms_new(R u, R Ds, R pmn2, R cdt, R f, R Dn) {
+    return ddiv(rfma(rmul(pmn2, cdt), f, rmul(u, Ds)), Dn);
+}
+
+// One phase of a substep on a strip of columns.  A warp owns the 29 columns i0 .. i0 + 28 (lane l is
+// column i0 + l - 2; lanes 0, 1 and 31 hold the neighbours) and walks up `nrows` rows from j0,
+// starting one row below for the free surface that the first row's V faces need.  West and east
+// neighbours come from the next lanes by shuffle, the southern ones from the row before, so a node's
+// inputs are loaded once (plus 3 columns in 32 and one row in nrows + 1), with no shared memory and no
+// barrier, and the new free surface is used by the momentum step from registers.
+//
+// The corrector also adds the fast-time averages, the predictor's terms (fields of level n, which
+// the substep does not change) and its own, in that order: one read and one write of the five FP64
+// averages per substep.  Neither phase reads a slot it writes (the predictor writes p and the
+// tendencies of level n, the corrector b), so warps are independent.
+//
+// Ring nodes of the free surface take the value of the nearest interior node (zero gradient at the
+// closed walls): its owner writes them.
+// Bound: bytes per node and substep 252 in FP32 (80 predictor, 172 corrector of which 80 the
+// averages), 404 in FP64.
+template <typename R>
+struct RomsRow {   // a node's inputs of one row
+    R z, h, v, om;                       // row j + 1: flux level's zeta and vbar, depth, om_v
+    R u, on, pm, pn, zk;                 // row j: flux level's ubar, metrics, zeta(kstp)
+    R fo, uk, vk, su, sv;                // row j, momentum only
+    R zrn, zrb, run, rub, rvn, rvb;      // corrector: tendencies of levels n and n-1
+};
+
+template <typename R, int PH>
+__device__ __forceinline__ void roms_load(const Geo<R> &g, const RomsArgs<R> &a, int il, int j, bool mom,
+                                          RomsRow<R> &w) {
+    const int J = g.J;
+    const int jc = j < 0 ? 0 : (j > J - 1 ? J - 1 : j);
+    const int jn = j + 1 < 0 ? 0 : (j + 1 > J - 1 ? J - 1 : j + 1);
+    const int p = jc * g.I + il, n = jn * g.I + il;
+    w.z = a.zrhs[n];
+    w.v = a.vrhs[n];
+    w.h = g.h[n];
+    w.om = g.om_v[n];
+    w.u = a.urhs[p];
+    w.on = g.on_u[p];
+    w.pm = g.pm[p];
+    w.pn = g.pn[p];
+    w.zk = a.zkstp[p];
+    w.fo = g.fomn[p];
+    if (PH == 1 && !a.first) {
+        w.zrn = a.rz_n[p];
+        w.zrb = a.rz_b[p];
+    }
+    if (mom) {
+        w.uk = a.ukstp[p];
+        w.vk = a.vkstp[p];
+        w.su = a.sustr[p];
+        w.sv = a.svstr[p];
+        if (PH == 1 && !a.first) {
+            w.run = a.ru_n[p];
+            w.rub = a.ru_b[p];
+            w.rvn = a.rv_n[p];
+            w.rvb = a.rv_b[p];
         }
     }
-    if (!a.step) return;
-    const int qi = i < 1 ? 1 : (i > g.I - 2 ? g.I - 2 : i);
-    const int qj = j < 1 ? 1 : (j > g.J - 2 ? g.J - 2 : j);
-    const long q = (long)qj * I + qi;
-    const R pmn = g.pm[q] * g.pn[q];
-    R znew;
-    if (a.phase == 0) {
-        const R rz = roms_rz(g, a.zn, a.un, a.vn, q, qi, qj);
-        const R cff1 = a.first ? (R)a.dtfast : (R)(2.0 * a.dtfast);
-        znew = a.zkstp[q] + (pmn * cff1) * rz;
-        if (q == p) a.rz_n[p] = rz;
-    } else {
-        const R rz = roms_rz(g, a.zp, a.up, a.vp, q, qi, qj);
-        const R dt = (R)a.dtfast;
-        if (a.first)
-            znew = a.zn[q] + (pmn * dt) * rz;
-        else
-            znew = a.zn[q] + (pmn * dt) * ((R(5.0 / 12.0) * rz + R(8.0 / 12.0) * a.rz_n[q]) -
-                                          R(1.0 / 12.0) * a.rz_b[q]);
+}
+
+template <typename R, int PH>
+__device__ __forceinline__ void roms_phase_rows(const Geo<R> &g, const RomsArgs<R> &a, const int i0,
+                                                const int j0, const int nrows) {
+    const int I = g.I, J = g.J, lane = threadIdx.x & 31;
+    if (j0 >= J) return;   // whole warp
+    const int i = i0 - 2 + lane, il = i < 0 ? 0 : (i > I - 1 ? I - 1 : i);
+    const bool out = lane >= 2 && lane <= 30 && i < I;
+    const int jend = j0 + nrows < J ? j0 + nrows : J;
+    auto west = [](R x) { return __shfl_up_sync(0xffffffffu, x, 1); };
+    auto east = [](R x) { return __shfl_down_sync(0xffffffffu, x, 1); };
+    const R rdrag2 = (R)a.rdrag2, dt = (R)a.dtfast;
+    const R dtz = PH == 0 && !a.first ? (R)(2.0 * a.dtfast) : dt;
+    const R cdt = PH == 0 && !a.first ? dt : (R)(0.5 * a.dtfast);
+    RomsRow<R> w;
+    // the row below the first: its southern values come from the load of the row before it
+    roms_load<R, PH>(g, a, il, j0 - 2, false, w);
+    R zc = w.z, hc = w.h, vc = w.v, omc = w.om;
+    R dvc, zks;   // DVom at row j; zeta(kstp) + h one row south
+    {
+        const int js = j0 - 2 < 0 ? 0 : j0 - 2;
+        const R Ds = a.zrhs[js * I + il] + g.h[js * I + il];
+        dvc = rmul(rmul(vc, rmul(R(0.5), (zc + hc) + Ds)), omc);
+        zks = R(0);
     }
-    a.zout[p] = znew;
-    if (a.phase == 0 && q != p) a.rz_n[p] = R(0);
+    R gs = R(0), hs = R(0), dzs = R(0), vfs = R(0), us = R(0), ues = R(0), pms = R(1), pns = R(1);
+    roms_load<R, PH>(g, a, il, j0 - 1, false, w);
+    for (int j = j0 - 1; j < jend; ++j) {
+        const RomsRow<R> c = w;
+        if (j + 1 < jend) roms_load<R, PH>(g, a, il, j + 1, true, w);   // the next row's, in flight
+        const bool mine = out && j >= j0;
+        const int p = j * I + i;
+        double A[5];
+        if (PH == 1 && a.acc == 1 && mine) {
+            A[0] = a.Zt[p];
+            A[1] = a.DU1[p];
+            A[2] = a.DV1[p];
+            A[3] = a.DU2[p];
+            A[4] = a.DV2[p];
+        }
+        // free surface
+        const R Dc = zc + hc, Dw = west(Dc);
+        const R au = rmul(c.u, rmul(R(0.5), Dc + Dw)), du = rmul(au, c.on);
+        const R dvn = rmul(rmul(c.v, rmul(R(0.5), (c.z + c.h) + Dc)), c.om);
+        const R rz = rfma(-east(au), east(c.on), du) + (dvc - dvn);
+        R f = rz;
+        if (PH == 1 && !a.first) f = roms_am3(rz, c.zrn, c.zrb);
+        const R znew = rfma(rmul(rmul(c.pm, c.pn), dtz), f, c.zk);
+        // the pressure-gradient surface
+        R gp;
+        if (a.first) gp = rmul(R(0.5), c.zk + znew);
+        else if (PH == 0) gp = rfma(R(0.68), zc, rmul(R(0.16), c.zk + znew));
+        else gp = rfma(R(0.6), znew, rmul(R(0.4), zc));
+        const R dk = c.zk + hc, dz = znew + hc;
+        const R ue = east(c.u);
+        const R fa = rmul(rmul(R(0.5), Dc), c.fo), vf = rmul(fa, c.u + ue);
+        if (j >= j0) {   // the whole warp
+            const bool ri = i >= 1 && i <= I - 2, rj = j >= 1 && j <= J - 2;
+            // U face
+            R unew = R(0), runew = R(0);
+            {
+                const R gw = west(gp), hw = west(hc);
+                const R cor = rfma(fa, vc + c.v, west(rmul(fa, vc + c.v)));
+                const R pmn2 = rmul(c.pm + west(c.pm), c.pn + west(c.pn));
+                const R v4 = rmul(R(0.25), ((vc + c.v) + west(vc)) + west(c.v));
+                const R Ds = dk + west(dk), Dn = dz + west(dz);
+                if (i >= 2 && ri && rj) {
+                    const R ru = roms_rhs<R, false>(c.on, gw, gp, hw, hc, cor, c.u, v4, rdrag2, c.su,
+                                                    ddiv(R(4.0), pmn2));
+                    R fu = ru;
+                    if (PH == 0) runew = ru;
+                    else if (!a.first) fu = roms_am3(ru, c.run, c.rub);
+                    unew = roms_new(c.uk, Ds, pmn2, cdt, fu, Dn);
+                }
+            }
+            // V face
+            R vnew = R(0), rvnew = R(0);
+            if (j >= 2 && rj && ri) {
+                const R pmn2 = rmul(c.pm + pms, c.pn + pns);
+                const R u4 = rmul(R(0.25), ((c.u + ue) + us) + ues);
+                const R rv = roms_rhs<R, true>(omc, gs, gp, hs, hc, rfma(fa, c.u + ue, vfs), vc, u4, rdrag2,
+                                               c.sv, ddiv(R(4.0), pmn2));
+                R fv = rv;
+                if (PH == 0) rvnew = rv;
+                else if (!a.first) fv = roms_am3(rv, c.rvn, c.rvb);
+                vnew = roms_new(c.vk, dk + zks, pmn2, cdt, fv, dz + dzs);
+            }
+            R dun = R(0), dvnn = R(0);
+            if (PH == 1 && a.acc) {   // DUon, DVom of level n (kstp): the predictor's terms
+                const R dkw = west(dk);
+                dun = i < 1 ? R(0) : rmul(rmul(c.uk, rmul(R(0.5), dk + dkw)), c.on);
+                dvnn = j < 1 ? R(0) : rmul(rmul(c.vk, rmul(R(0.5), dk + zks)), omc);
+            }
+            if (mine) {
+                a.uout[p] = unew;
+                a.vout[p] = vnew;
+                if (PH == 0) {
+                    a.ru_n[p] = runew;
+                    a.rv_n[p] = rvnew;
+                    a.rz_n[p] = ri && rj ? rz : R(0);
+                }
+                if (ri && rj) {
+                    const int di = i == 1 ? -1 : (i == I - 2 ? 1 : 0), dj = j == 1 ? -I : (j == J - 2 ? I : 0);
+                    a.zout[p] = znew;
+                    if (di) a.zout[p + di] = znew;
+                    if (dj) a.zout[p + dj] = znew;
+                    if (di && dj) a.zout[p + di + dj] = znew;
+                }
+                if (PH == 1 && a.acc) {
+                    const double dun_ = (double)dun, dvn_ = (double)dvnn;
+                    const double dup = i < 1 ? 0.0 : (double)du, dvp = j < 1 ? 0.0 : (double)dvc;
+                    if (a.acc == 2) {
+                        A[0] = 0.0;
+                        A[1] = 0.0;
+                        A[2] = 0.0;
+                        A[3] = __dmul_rn(a.c2, dun_);
+                        A[4] = __dmul_rn(a.c2, dvn_);
+                    } else {
+                        A[0] = rsum<R>(A[0], a.c1, (double)c.zk);
+                        A[1] = rsum<R>(A[1], a.c1, dun_);
+                        A[2] = rsum<R>(A[2], a.c1, dvn_);
+                        A[3] = rsum<R>(A[3], a.c2, dun_);
+                        A[4] = rsum<R>(A[4], a.c2, dvn_);
+                    }
+                    a.Zt[p] = A[0];
+                    a.DU1[p] = A[1];
+                    a.DV1[p] = A[2];
+                    a.DU2[p] = rsum<R>(A[3], a.c2c, dup);
+                    a.DV2[p] = rsum<R>(A[4], a.c2c, dvp);
+                }
+            }
+        }
+        // this row becomes the southern one
+        gs = gp;
+        hs = hc;
+        zks = dk;
+        dzs = dz;
+        vfs = vf;
+        us = c.u;
+        ues = ue;
+        pms = c.pm;
+        pns = c.pn;
+        dvc = dvn;
+        zc = c.z;
+        hc = c.h;
+        vc = c.v;
+        omc = c.om;
+    }
 }
 
-// The pressure-gradient surface zwrk of a phase at rho q (zout holds the phase's new zeta).
-template <typename R>
-__device__ __forceinline__ R roms_zwrk(const RomsArgs<R> &a, long q) {
-    const R znew = a.zout[q];
-    if (a.first) return R(0.5) * (a.zkstp[q] + znew);
-    if (a.phase == 0) return R(0.68) * a.zn[q] + R(0.16) * (a.zkstp[q] + znew);
-    return R(0.6) * znew + R(0.4) * a.zp[q];
+// A whole leapfrog / AM3 substep (predictor and corrector, free surface and momentum) in one launch.
+// A block of 32 x H threads stages 32 columns (27 of them its own: lanes 3..29) and H rows (H - 3 its
+// own: warps 2 .. H - 2), one node per thread.  Every node's inputs are loaded at once; the four
+// stages then follow with x-neighbours by shuffle, y-neighbours through shared memory and three
+// barriers, the halo nodes computing again what their owners compute.  Per substep and node 172
+// bytes in FP32 (levels n and n-1, metrics, stresses and tendencies read once, level n+1 and the
+// tendencies written, 80 bytes of FP64 averages) against 252 in two launches, and one launch
+// latency, which is what small grids pay for.
+//
+// Level n+1 goes to the scratch slot (zout, uout, vout = slot p), because other blocks still read
+// slot b at their halos; the host rotates the three slots.
+// A copy of one value of the thread's own into its own shared-memory word: in flight without
+// holding a register until it is read (after cp_own_wait).
+template <typename T>
+__device__ __forceinline__ void cp_own(T *dst, const T *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(sizeof(T))
+                 : "memory");
+}
+__device__ __forceinline__ void cp_own_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_own_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-// Momentum of a phase at the U and V faces of p (0 on walls and the ring).
+template <typename R, int H, bool LATE>
+__device__ __forceinline__ void roms_sub_tile(const Geo<R> &g, const RomsArgs<R> &a, const int i0,
+                                              const int j0, unsigned char *raw) {
+    const int I = g.I, J = g.J, lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+    const int i = i0 - 3 + lane, j = j0 - 2 + wy;
+    const int il = i < 0 ? 0 : (i > I - 1 ? I - 1 : i), jl = j < 0 ? 0 : (j > J - 1 ? J - 1 : j);
+    const int js = j - 1 < 0 ? 0 : (j - 1 > J - 1 ? J - 1 : j - 1);
+    const int jn = j + 1 < 0 ? 0 : (j + 1 > J - 1 ? J - 1 : j + 1);
+    const int q = jl * I + il, qs = js * I + il, qn = jn * I + il;
+    const bool ri = i >= 1 && i <= I - 2, rj = j >= 1 && j <= J - 2;
+    const bool uface = i >= 2 && ri && rj, vface = j >= 2 && rj && ri;
+    const bool mine = lane >= 3 && lane <= 29 && i < I && wy >= 2 && wy <= H - 2 && j < J;
+    auto west = [](R x) { return __shfl_up_sync(0xffffffffu, x, 1); };
+    auto east = [](R x) { return __shfl_down_sync(0xffffffffu, x, 1); };
+    const R rdrag2 = (R)a.rdrag2, dt = (R)a.dtfast, dt2 = (R)(2.0 * a.dtfast), dth = (R)(0.5 * a.dtfast);
+    // the context's metrics do not depend on the kernels before: loaded while those finish
+    const R h = g.h[q], hs = g.h[qs], hn = g.h[qn], om = g.om_v[q], omN = g.om_v[qn];
+    const R on = g.on_u[q], pm = g.pm[q], pn = g.pn[q], fo = g.fomn[q];
+    pdl_wait_then_launch();
+    // LATE: values needed late wait in shared memory (averages; the old level's velocities, stresses,
+    // tendencies), which leaves registers for more blocks per SM; else in registers
+    constexpr int T = 32 * H;
+    double *const av = reinterpret_cast<double *>(raw) + threadIdx.x;
+    R *const own = reinterpret_cast<R *>(raw + 5 * T * sizeof(double)) + threadIdx.x;
+    R *const sm = reinterpret_cast<R *>(raw + (LATE ? T * (5 * sizeof(double) + 7 * sizeof(R)) : 0)) + 32;
+    // level n at the node and its row neighbours
+    const R zn = a.zrhs[q], un = a.urhs[q], vn = a.vrhs[q];
+    const R zs_ = a.zrhs[qs], zn_ = a.zrhs[qn], vN = a.vrhs[qn], zb = a.zkstp[q];
+    const R *const lp[7] = {a.ukstp, a.vkstp, a.sustr, a.svstr, a.rz_b, a.ru_b, a.rv_b};
+    double *const ap[5] = {a.Zt, a.DU1, a.DV1, a.DU2, a.DV2};
+    enum { UB, VB, SU, SV, RZB, RUB, RVB };
+    R lr[7];
+    double ar[5];
+#pragma unroll
+    for (int f = 0; f < 7; ++f) {
+        if constexpr (LATE) cp_own(own + f * T, lp[f] + q);
+        else lr[f] = lp[f][q];
+    }
+    if constexpr (LATE) cp_own_commit();
+    if (a.acc && mine) {
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+            if constexpr (LATE) cp_own(av + f * T, ap[f] + q);
+            else ar[f] = ap[f][q];
+        }
+    }
+    if constexpr (LATE) cp_own_commit();
+    auto late = [&](int f) -> R {
+        if constexpr (LATE) return own[f * T];
+        else return lr[f];
+    };
+    auto avg = [&](int f) -> double {
+        if constexpr (LATE) return av[f * T];
+        else return ar[f];
+    };
+    constexpr int S = T;   // one exchanged field
+    R *const me = sm + threadIdx.x;
+    enum { GP, DK, VF, U, PM, PN, DZ, VP };
+#define SF_SOUTH(f) me[(f) * S - 32]
+#define SF_NORTH(f) me[(f) * S + 32]
+    // rows 0 and H - 1 have no southern / northern neighbour in the block: what is then read lies in
+    // the neighbouring field (or the pad before the first) and reaches no owned node
+    // predictor: free surface
+    const R D = zn + h, Ds = zs_ + hs, Dn = zn_ + hn;
+    const R onE = east(on), pmn = rmul(pm, pn);
+    const R au = rmul(un, rmul(R(0.5), D + west(D))), du = rmul(au, on);
+    const R dv = rmul(rmul(vn, rmul(R(0.5), D + Ds)), om);
+    const R dvN = rmul(rmul(vN, rmul(R(0.5), Dn + D)), omN);
+    const R rz = rfma(-east(au), onE, du) + (dv - dvN);
+    const R zp = rfma(rmul(pmn, dt2), rz, zb);
+    R gp = rfma(R(0.68), zn, rmul(R(0.16), zb + zp));
+    const R dk = zb + h, dz = zp + h, ue = east(un);
+    R fa = rmul(rmul(R(0.5), D), fo), vf = rmul(fa, un + ue);
+    me[GP * S] = gp;
+    me[DK * S] = dk;
+    me[VF * S] = vf;
+    me[U * S] = un;
+    me[PM * S] = pm;
+    me[PN * S] = pn;
+    me[DZ * S] = dz;
+    __syncthreads();
+    // predictor: momentum (not on row 0, nor U faces on row H - 1: no owned node needs them)
+    if constexpr (LATE) cp_own_wait<1>();
+    const R hw = west(h), pmw = rmul(pm + west(pm), pn + west(pn));
+    const R pms = rmul(pm + SF_SOUTH(PM), pn + SF_SOUTH(PN));
+    const R areaU = ddiv(R(4.0), pmw), areaV = ddiv(R(4.0), pms);
+    R up = R(0), vp = R(0), ru = R(0), rv = R(0);
+    if (wy > 0) {
+        const R gw = west(gp), cor = rfma(fa, vn + vN, west(rmul(fa, vn + vN)));
+        const R v4 = rmul(R(0.25), ((vn + vN) + west(vn)) + west(vN));
+        const R dkw = dk + west(dk), dzw = dz + west(dz);
+        if (uface && wy < H - 1) {
+            ru = roms_rhs<R, false>(on, gw, gp, hw, h, cor, un, v4, rdrag2, late(SU), areaU);
+            up = roms_new(late(UB), dkw, pmw, dt, ru, dzw);
+        }
+        if (vface) {
+            const R u4 = rmul(R(0.25), ((un + ue) + SF_SOUTH(U)) + me[U * S - 31]);
+            rv = roms_rhs<R, true>(om, SF_SOUTH(GP), gp, hs, h, rfma(fa, un + ue, SF_SOUTH(VF)), vn, u4,
+                                   rdrag2, late(SV), areaV);
+            vp = roms_new(late(VB), dk + SF_SOUTH(DK), pms, dt, rv, dz + SF_SOUTH(DZ));
+        }
+    }
+    me[VP * S] = vp;
+    __syncthreads();
+    // corrector: free surface (rows 1 .. H - 2)
+    R vpN = R(0), upE = R(0), dup = R(0), dvp = R(0), zc = R(0), dzc = R(0);
+    if (wy > 0 && wy < H - 1) {
+        vpN = SF_NORTH(VP);
+        upE = east(up);
+        const R aup = rmul(up, rmul(R(0.5), dz + west(dz)));
+        dup = rmul(aup, on);
+        dvp = rmul(rmul(vp, rmul(R(0.5), dz + SF_SOUTH(DZ))), om);
+        const R dvpN = rmul(rmul(vpN, rmul(R(0.5), SF_NORTH(DZ) + dz)), omN);
+        const R rzc = rfma(-east(aup), onE, dup) + (dvp - dvpN);
+        zc = rfma(rmul(pmn, dt), roms_am3(rzc, rz, late(RZB)), zn);
+        gp = rfma(R(0.6), zc, rmul(R(0.4), zp));
+        dzc = zc + h;
+        fa = rmul(rmul(R(0.5), dz), fo);
+        vf = rmul(fa, up + upE);
+        me[GP * S] = gp;   // the predictor's values of these fields were read before the last barrier
+        me[DK * S] = dzc;
+        me[VF * S] = vf;
+        me[U * S] = up;
+    }
+    __syncthreads();
+    if (wy < 2 || wy > H - 2) return;
+    // corrector: momentum (the owned rows)
+    R uc = R(0), vc = R(0);
+    {
+        const R gw = west(gp), cor = rfma(fa, vp + vpN, west(rmul(fa, vp + vpN)));
+        const R v4 = rmul(R(0.25), ((vp + vpN) + west(vp)) + west(vpN));
+        const R Dw = D + west(D), dzw = dzc + west(dzc);
+        if (uface) {
+            const R r = roms_rhs<R, false>(on, gw, gp, hw, h, cor, up, v4, rdrag2, late(SU), areaU);
+            uc = roms_new(un, Dw, pmw, dth, roms_am3(r, ru, late(RUB)), dzw);
+        }
+        if (vface) {
+            const R u4 = rmul(R(0.25), ((up + upE) + SF_SOUTH(U)) + me[U * S - 31]);
+            const R r = roms_rhs<R, true>(om, SF_SOUTH(GP), gp, hs, h, rfma(fa, up + upE, SF_SOUTH(VF)), vp, u4,
+                                          rdrag2, late(SV), areaV);
+            vc = roms_new(vn, D + Ds, pms, dth, roms_am3(r, rv, late(RVB)), dzc + SF_SOUTH(DK));
+        }
+    }
+#undef SF_SOUTH
+#undef SF_NORTH
+    if (!mine) return;
+    a.uout[q] = uc;
+    a.vout[q] = vc;
+    a.ru_n[q] = ru;
+    a.rv_n[q] = rv;
+    a.rz_n[q] = ri && rj ? rz : R(0);
+    if (ri && rj) {   // the free surface, and the ring nodes next to it
+        const int di = i == 1 ? -1 : (i == I - 2 ? 1 : 0), dj = j == 1 ? -I : (j == J - 2 ? I : 0);
+        a.zout[q] = zc;
+        if (di) a.zout[q + di] = zc;
+        if (dj) a.zout[q + dj] = zc;
+        if (di && dj) a.zout[q + di + dj] = zc;
+    }
+    if (a.acc) {
+        if constexpr (LATE) cp_own_wait<0>();
+        const double un1 = i < 1 ? 0.0 : (double)du, vn1 = j < 1 ? 0.0 : (double)dv;
+        const double up1 = i < 1 ? 0.0 : (double)dup, vp1 = j < 1 ? 0.0 : (double)dvp;
+        a.Zt[q] = rsum<R>(avg(0), a.c1, (double)zn);
+        a.DU1[q] = rsum<R>(avg(1), a.c1, un1);
+        a.DV1[q] = rsum<R>(avg(2), a.c1, vn1);
+        a.DU2[q] = rsum<R>(rsum<R>(avg(3), a.c2, un1), a.c2c, up1);
+        a.DV2[q] = rsum<R>(rsum<R>(avg(4), a.c2, vn1), a.c2c, vp1);
+    }
+}
+
+// The fast-time averages of the loop's last substep (nfast + 1), which only accumulates the fields
+// of level n (step2d_LF_AM3.h.py:923-926).
 template <typename R>
-__device__ __forceinline__ void roms_mom_at(const Geo<R> &g, const RomsArgs<R> &a, const long p) {
+__device__ __forceinline__ void roms_acc_at(const Geo<R> &g, const RomsArgs<R> &a, const long p) {
     if (p >= g.s2) return;
     const int j = fdiv((int)p, g.dI), i = (int)p - j * g.I;
-    const long I = g.I;
-    const R *h = g.h;
-    const R cffg = R(0.5 * 10.0);                    // 0.5 g, g = 10 (mod_constants.py:26)
-    const R *zr = a.zrhs, *ur = a.urhs, *vr = a.vrhs;
-    const R rdrag2 = (R)a.rdrag2;
-    const R cdt = a.first ? (R)(0.5 * a.dtfast) : (a.phase == 0 ? (R)a.dtfast : (R)(0.5 * a.dtfast));
-    // U face p
-    R unew = R(0), runew = R(0);
-    if (i >= 2 && i <= g.I - 2 && j >= 1 && j <= g.J - 2) {
-        const R gp = roms_zwrk(a, p), gw = roms_zwrk(a, p - 1);
-        const R gp2 = gp * gp, gw2 = gw * gw;
-        const R pg = (cffg * g.on_u[p]) * ((h[p - 1] + h[p]) * (gw - gp) + (gw2 - gp2));
-        const R UFp = ((R(0.5) * (zr[p] + h[p])) * g.fomn[p]) * (vr[p] + vr[p + I]);
-        const R UFw = ((R(0.5) * (zr[p - 1] + h[p - 1])) * g.fomn[p - 1]) * (vr[p - 1] + vr[p - 1 + I]);
-        const R cor = R(0.5) * (UFp + UFw);
-        const R area = ddiv(R(4.0), (g.pm[p] + g.pm[p - 1]) * (g.pn[p] + g.pn[p - 1]));
-        const R v4 = R(0.25) * (((vr[p] + vr[p + I]) + vr[p - 1]) + vr[p - 1 + I]);
-        const R ub = ur[p];
-        const R bustr = (rdrag2 * ub) * sqrt(ub * ub + v4 * v4);
-        const R ru = (pg + cor) + (a.sustr[p] - bustr) * area;
-        R f = ru;
-        if (a.phase == 0) runew = ru;
-        else if (!a.first) f = (R(5.0 / 12.0) * ru + R(8.0 / 12.0) * a.ru_n[p]) - R(1.0 / 12.0) * a.ru_b[p];
-        const R cff = (g.pm[p] + g.pm[p - 1]) * (g.pn[p] + g.pn[p - 1]);
-        const R Ds = (a.zkstp[p] + h[p]) + (a.zkstp[p - 1] + h[p - 1]);
-        const R Dn = (a.zout[p] + h[p]) + (a.zout[p - 1] + h[p - 1]);
-        unew = ddiv(a.ukstp[p] * Ds + (cff * cdt) * f, Dn);
-    }
-    a.uout[p] = unew;
-    if (a.phase == 0) a.ru_n[p] = runew;
-    // V face p
-    R vnew = R(0), rvnew = R(0);
-    if (j >= 2 && j <= g.J - 2 && i >= 1 && i <= g.I - 2) {
-        const R gp = roms_zwrk(a, p), gs = roms_zwrk(a, p - I);
-        const R gp2 = gp * gp, gs2 = gs * gs;
-        const R pg = (cffg * g.om_v[p]) * ((h[p - I] + h[p]) * (gs - gp) + (gs2 - gp2));
-        const R VFp = ((R(0.5) * (zr[p] + h[p])) * g.fomn[p]) * (ur[p] + ur[p + 1]);
-        const R VFs = ((R(0.5) * (zr[p - I] + h[p - I])) * g.fomn[p - I]) * (ur[p - I] + ur[p - I + 1]);
-        const R cor = R(-0.5) * (VFp + VFs);
-        const R area = ddiv(R(4.0), (g.pm[p] + g.pm[p - I]) * (g.pn[p] + g.pn[p - I]));
-        const R u4 = R(0.25) * (((ur[p] + ur[p + 1]) + ur[p - I]) + ur[p - I + 1]);
-        const R vb = vr[p];
-        const R bvstr = (rdrag2 * vb) * sqrt(u4 * u4 + vb * vb);
-        const R rv = (pg + cor) + (a.svstr[p] - bvstr) * area;
-        R f = rv;
-        if (a.phase == 0) rvnew = rv;
-        else if (!a.first) f = (R(5.0 / 12.0) * rv + R(8.0 / 12.0) * a.rv_n[p]) - R(1.0 / 12.0) * a.rv_b[p];
-        const R cff = (g.pm[p] + g.pm[p - I]) * (g.pn[p] + g.pn[p - I]);
-        const R Ds = (a.zkstp[p] + h[p]) + (a.zkstp[p - I] + h[p - I]);
-        const R Dn = (a.zout[p] + h[p]) + (a.zout[p - I] + h[p - I]);
-        vnew = ddiv(a.vkstp[p] * Ds + (cff * cdt) * f, Dn);
-    }
-    a.vout[p] = vnew;
-    if (a.phase == 0) a.rv_n[p] = rvnew;
+    const R *z = a.zrhs, *h = g.h;
+    const R D = z[p] + h[p];
+    double du = 0.0, dv = 0.0;
+    if (i >= 1) du = (double)rmul(rmul(a.urhs[p], rmul(R(0.5), D + (z[p - 1] + h[p - 1]))), g.on_u[p]);
+    if (j >= 1) dv = (double)rmul(rmul(a.vrhs[p], rmul(R(0.5), D + (z[p - g.I] + h[p - g.I]))), g.om_v[p]);
+    a.Zt[p] = rsum<R>(a.Zt[p], a.c1, (double)z[p]);
+    a.DU1[p] = rsum<R>(a.DU1[p], a.c1, du);
+    a.DV1[p] = rsum<R>(a.DV1[p], a.c1, dv);
+    a.DU2[p] = rsum<R>(a.DU2[p], a.c2, du);
+    a.DV2[p] = rsum<R>(a.DV2[p], a.c2, dv);
 }
 
 // The ROMS-form 3D momentum right-hand side at the interior faces (U: j = 1..J-2, i = 2..I-2;
@@ -445,12 +773,9 @@ __device__ __forceinline__ T *at(T *x, long o) { return x ? x + o : x; }
 template <typename R>
 __device__ __forceinline__ RomsArgs<R> roms_args_at(const RomsArgs<R> &a, long o) {
     RomsArgs<R> b = a;
-    b.zb = at(a.zb, o); b.zn = at(a.zn, o); b.zp = at(a.zp, o);
-    b.ub = at(a.ub, o); b.un = at(a.un, o); b.up = at(a.up, o);
-    b.vb = at(a.vb, o); b.vn = at(a.vn, o); b.vp = at(a.vp, o);
-    b.zout = at(a.zout, o); b.uout = at(a.uout, o); b.vout = at(a.vout, o);
-    b.zkstp = at(a.zkstp, o); b.ukstp = at(a.ukstp, o); b.vkstp = at(a.vkstp, o);
     b.zrhs = at(a.zrhs, o); b.urhs = at(a.urhs, o); b.vrhs = at(a.vrhs, o);
+    b.zkstp = at(a.zkstp, o); b.ukstp = at(a.ukstp, o); b.vkstp = at(a.vkstp, o);
+    b.zout = at(a.zout, o); b.uout = at(a.uout, o); b.vout = at(a.vout, o);
     b.rz_n = at(a.rz_n, o); b.ru_n = at(a.ru_n, o); b.rv_n = at(a.rv_n, o);
     b.rz_b = at(a.rz_b, o); b.ru_b = at(a.ru_b, o); b.rv_b = at(a.rv_b, o);
     b.sustr = at(a.sustr, o); b.svstr = at(a.svstr, o);
@@ -459,30 +784,74 @@ __device__ __forceinline__ RomsArgs<R> roms_args_at(const RomsArgs<R> &a, long o
     return b;
 }
 
-// The barotropic phases are launched with programmatic dependent launch (as the reference
-// form's loop): a kernel's blocks become resident while its predecessor's last wave runs and
-// wait for its completion on the device (pdl_enter) before touching any field.
-template <typename R>
-__global__ void __launch_bounds__(256) k_roms_zeta(Geo<R> g, RomsArgs<R> a) {
-    pdl_enter();
-    roms_zeta_at(g, a, tid_flat());
+template <typename R, int PH>
+__global__ void __launch_bounds__(32 * kRomsWarps) k_roms_phase(Geo<R> g, RomsArgs<R> a, int nrows) {
+    pdl_wait_then_launch();
+    roms_phase_rows<R, PH>(g, a, (int)blockIdx.x * kRomsCols,
+                           ((int)blockIdx.y * kRomsWarps + (int)(threadIdx.x >> 5)) * nrows, nrows);
+}
+template <typename R, int PH>
+__global__ void __launch_bounds__(32 * kRomsWarps) kb_roms_phase(const Member<R> *mt, const int2 *bm,
+                                                                 RomsArgs<R> a, int nrows) {
+    pdl_wait_then_launch();
+    const int2 mb = bm[blockIdx.x];
+    const Member<R> &M = mt[mb.x];
+    const int ns = (M.g.I + kRomsCols - 1) / kRomsCols, by = mb.y / ns, bx = mb.y - by * ns;
+    roms_phase_rows<R, PH>(M.g, roms_args_at(a, M.off2), bx * kRomsCols,
+                           (by * kRomsWarps + (int)(threadIdx.x >> 5)) * nrows, nrows);
+}
+// Shared memory of a block: per node (LATE) 5 averages and 7 late inputs, 8 exchanged values, and a
+// row of pad on either side of the exchanged fields.
+template <typename R, bool LATE>
+constexpr int roms_sub_smem(int H) {
+    return (LATE ? 32 * H * (40 + 7 * (int)sizeof(R)) : 0) + (8 * H + 2) * 32 * (int)sizeof(R);
+}
+// Blocks per SM the register cap allows for: LATE in FP32 3 of 384 threads at 56 registers (4 at 40
+// spill: 2050 x 1026 loop 5.10 against 4.35 ms), in FP64 2 at 80; else uncapped.
+template <typename R, bool LATE>
+constexpr int roms_sub_blocks() { return !LATE ? 1 : (sizeof(R) == 4 ? 3 : 2); }
+template <typename R, int H, bool LATE>
+__global__ void __launch_bounds__(32 * H, roms_sub_blocks<R, LATE>()) k_roms_sub(Geo<R> g, RomsArgs<R> a) {
+    extern __shared__ __align__(16) unsigned char sub_smem[];
+    roms_sub_tile<R, H, LATE>(g, a, (int)blockIdx.x * kSubCols, (int)blockIdx.y * (H - 3), sub_smem);
+}
+template <typename R, int H, bool LATE>
+__global__ void __launch_bounds__(32 * H, roms_sub_blocks<R, LATE>()) kb_roms_sub(const Member<R> *mt, const int2 *bm,
+                                                                               RomsArgs<R> a) {
+    extern __shared__ __align__(16) unsigned char sub_smem[];
+    const int2 mb = bm[blockIdx.x];
+    const Member<R> &M = mt[mb.x];
+    const int ns = (M.g.I + kSubCols - 1) / kSubCols, by = mb.y / ns, bx = mb.y - by * ns;
+    roms_sub_tile<R, H, LATE>(M.g, roms_args_at(a, M.off2), bx * kSubCols, by * (H - 3), sub_smem);
+}
+template <typename R, bool LATE>
+cudaError_t roms_sub_launch(const sf_ctx *c, const RomsArgs<R> &a, dim3 grid, cudaStream_t s) {
+    constexpr int H = kSubRows, smem = roms_sub_smem<R, LATE>(H);
+    static bool done[64] = {};   // the raised shared-memory limit, once on each device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+        const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        e = cudaFuncSetAttribute(k_roms_sub<R, H, LATE>, at, smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kb_roms_sub<R, H, LATE>, at, smem);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) done[dev] = true;
+    }
+    if (c->nmem > 1)
+        return launch_dep(c, kb_roms_sub<R, H, LATE>, grid, 32 * H, smem, s, mt<R>(c), c->bm_sub, a);
+    return launch_dep(c, k_roms_sub<R, H, LATE>, grid, 32 * H, smem, s, Ops<R>::geo(c), a);
 }
 template <typename R>
-__global__ void __launch_bounds__(256) kb_roms_zeta(const Member<R> *mt, const int2 *bm, RomsArgs<R> a) {
-    pdl_enter();
+__global__ void __launch_bounds__(256) k_roms_acc(Geo<R> g, RomsArgs<R> a) {
+    pdl_wait_then_launch();
+    roms_acc_at(g, a, tid_flat());
+}
+template <typename R>
+__global__ void __launch_bounds__(256) kb_roms_acc(const Member<R> *mt, const int2 *bm, RomsArgs<R> a) {
+    pdl_wait_then_launch();
     const MemberAt<R> m = member_at(mt, bm, 256);
-    roms_zeta_at(m.g, roms_args_at(a, m.o2), m.p);
-}
-template <typename R>
-__global__ void __launch_bounds__(256) k_roms_mom(Geo<R> g, RomsArgs<R> a) {
-    pdl_enter();
-    roms_mom_at(g, a, tid_flat());
-}
-template <typename R>
-__global__ void __launch_bounds__(256) kb_roms_mom(const Member<R> *mt, const int2 *bm, RomsArgs<R> a) {
-    pdl_enter();
-    const MemberAt<R> m = member_at(mt, bm, 256);
-    roms_mom_at(m.g, roms_args_at(a, m.o2), m.p);
+    roms_acc_at(m.g, roms_args_at(a, m.o2), m.p);
 }
 template <typename R>
 __global__ void __launch_bounds__(256) k_roms_rhs3d(Geo<R> g, const R *u, const R *v, const R *Hu,
@@ -552,15 +921,28 @@ __global__ void __launch_bounds__(256) kb_roms_walls3d(const Member<R> *mt, cons
 
 template <typename R>
 cudaError_t Ops<R>::roms_phase(const sf_ctx *c, const RomsArgs<R> &a, cudaStream_t s) {
-    if (c->nmem > 1) {
-        cudaError_t e = launch_dep(c, kb_roms_zeta<R>, c->nbm_pt, 256, 0, s, mt<R>(c), c->bm_pt, a);
-        if (e != cudaSuccess || !a.step) return e;
-        return launch_dep(c, kb_roms_mom<R>, c->nbm_pt, 256, 0, s, mt<R>(c), c->bm_pt, a);
+    const int B = 32 * kRomsWarps;
+    if (a.phase == 3) {
+        dim3 grid((c->I + kSubCols - 1) / kSubCols, (c->J + kSubRows - 4) / (kSubRows - 3));
+        if (c->nmem > 1) grid = dim3(c->nbm_sub);
+        // few tiles: one node's latency counts, everything in registers (514 x 258 nodes, 580 tiles, FP32:
+        // 367 us a loop of 52 substeps against 437; 130 x 66, FP64: 220 against 229); many: blocks per
+        // SM count (642 x 322, 864 tiles, FP32: 480 against 512; 514 x 258, FP64: 638 against 716; at
+        // 258 x 130, 150 tiles, FP64 takes 333 and 336)
+        return (long)grid.x * grid.y >= (sizeof(R) == 4 ? 720 : 200) ? roms_sub_launch<R, true>(c, a, grid, s)
+                                                                     : roms_sub_launch<R, false>(c, a, grid, s);
     }
-    const unsigned nb = blocks_for(c->s2, 256);
-    cudaError_t e = launch_dep(c, k_roms_zeta<R>, nb, 256, 0, s, geo(c), a);
-    if (e != cudaSuccess || !a.step) return e;
-    return launch_dep(c, k_roms_mom<R>, nb, 256, 0, s, geo(c), a);
+    if (c->nmem > 1) {
+        if (a.phase == 2)
+            return launch_dep(c, kb_roms_acc<R>, c->nbm_pt, 256, 0, s, mt<R>(c), c->bm_pt, a);
+        auto k = a.phase == 0 ? kb_roms_phase<R, 0> : kb_roms_phase<R, 1>;
+        return launch_dep(c, k, c->nbm_roms, B, 0, s, mt<R>(c), c->bm_roms, a, c->roms_rows);
+    }
+    if (a.phase == 2) return launch_dep(c, k_roms_acc<R>, blocks_for(c->s2, 256), 256, 0, s, geo(c), a);
+    const int rows = c->roms_rows;
+    const dim3 grid((c->I + kRomsCols - 1) / kRomsCols, (c->J + rows * kRomsWarps - 1) / (rows * kRomsWarps));
+    auto k = a.phase == 0 ? k_roms_phase<R, 0> : k_roms_phase<R, 1>;
+    return launch_dep(c, k, grid, B, 0, s, geo(c), a, rows);
 }
 template <typename R>
 cudaError_t Ops<R>::roms_stress3d(const sf_ctx *c, const R *u, const R *v, R *ru, R *rv,

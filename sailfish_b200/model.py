@@ -245,6 +245,14 @@ class Model:
         if rdrag2 is not None:
             self.rdrag2 = float(rdrag2)
 
+    @property
+    def loop_launches(self):
+        """Kernel launches of the ROMS-form barotropic loop: of its nfast substeps the first and the
+        last one to six take two, the groups of six between them one each (fused); one more for
+        the averages of substep nfast + 1."""
+        fused = max(0, self.nfast - 2) // 6 * 6
+        return 2 * (self.nfast - fused) + fused + 1
+
     def _roms_loop(self, s, stream):
         W1 = self.W1.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
         W2 = self.W2.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
@@ -259,15 +267,19 @@ class Model:
         if self.semantics != "roms":
             raise ValueError("step2d is the ROMS-form 2D driver (semantics='roms')")
         st = stream_handle()
-        for _ in range(nsteps):
-            f = (not getattr(self, "_started2d", False)) if first is None else first
+        if first is None:   # one call for the run of steps
+            runs = [(nsteps, not getattr(self, "_started2d", False))] if nsteps > 0 else []
+        else:
+            runs = [(1, first)] * nsteps
+        for n, f in runs:
             s = self.state2d()
-            check(lib.sf_roms_step2d(self.ctx.ptr, ctypes.byref(s), self._p(self.sustr),
-                                     self._p(self.svstr), self.rdrag2, self.dtfast, int(f), st),
-                  "sf_roms_step2d")
+            check(lib.sf_roms_steps2d(self.ctx.ptr, ctypes.byref(s), self._p(self.sustr),
+                                      self._p(self.svstr), self.rdrag2, self.dtfast, n, int(f), st),
+                  "sf_roms_steps2d")
             self._sync_slots(s)
             self._started2d = True
-            self.time2D += self.dtfast
+            for _ in range(n):
+                self.time2D += self.dtfast
 
     # -- steps -------------------------------------------------------------------------------
     def check_state(self, stream=None):
