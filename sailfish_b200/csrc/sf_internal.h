@@ -2,6 +2,7 @@
 // (sf_kernels_f64.cu, sf_kernels_f32.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <type_traits>
 #include <stdint.h>
 
 #include "../../include/sailfish_b200.h"

@@ -592,122 +592,170 @@ __device__ __forceinline__ void roms_stress3d_at(const Geo<R> &g, const R *__res
 // vertical advection).  Thomas elimination in R, then the depth mean set to the barotropic
 // transport with FP64 sums: x_k -= (sum Hzu x - avg/on) / sum Hzu.  Returns the new depth-mean
 // velocity avg/on/sum Hzu.
+// Bound: latency of the level loads at 12 to 16 warps per SM (56 bytes a point and component pair in
+// FP32, 1.4 GB and 0.21 ms at the copy bandwidth for 1003 x 501 x 50; 0.82 ms before with per-thread
+// local arrays and U and V columns half a grid apart, 0.45 now).
 template <typename R>
 struct RomsRhs {
     const R *r0, *r1, *r2;   // right-hand sides at n, n-1, n-2
 };
 
+// Levels whose loads the column solve issues together (1003 x 501 x 50, FP32: 2, 4, 6, 8, 12 levels 0.59,
+// 0.59, 0.47, 0.45, 0.53 ms, 118 to 197 registers; FP64 4, 6, 8: 1.29, 1.27, 1.33).
 template <typename R>
-__device__ __forceinline__ double roms_column(const Geo<R> &g, long p, long d, R *__restrict__ u,
-                                              RomsRhs<R> rs, R c0, R c1, R c2,
-                                              const R *__restrict__ Hz,
+constexpr int roms_col_chunk() { return sizeof(R) == 4 ? 8 : 6; }
+// f(C) for n levels in chunks of C, what is left in chunks of 4, 2 and 1
+template <int C, typename F>
+__device__ __forceinline__ void in_chunks(int n, F f) {
+    for (; n >= C; n -= C) f(std::integral_constant<int, C>());
+    if (n >= 4) {
+        f(std::integral_constant<int, 4>());
+        n -= 4;
+    }
+    if (n >= 2) {
+        f(std::integral_constant<int, 2>());
+        n -= 2;
+    }
+    if (n >= 1) f(std::integral_constant<int, 1>());
+}
+// A pivot of the elimination as its divisions use it: in FP32 the reciprocal (a / b through
+// __fdividef is a times the hardware reciprocal of b, bit for bit in b's normal range, and every
+// pivot divides twice), in FP64 the pivot itself (IEEE division).
+__device__ __forceinline__ float roms_pivot(float b) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return r;
+}
+__device__ __forceinline__ double roms_pivot(double b) { return b; }
+__device__ __forceinline__ float over_pivot(float a, float r) { return __fmul_rn(a, r); }
+__device__ __forceinline__ double over_pivot(double a, double b) { return a / b; }
+// a / b, its last product not fused into a sum that takes it
+template <typename R>
+__device__ __forceinline__ R roms_div(R a, R b) { return over_pivot(a, roms_pivot(b)); }
+
+// Per column two arrays in shared memory, [level][thread]: the pivots, overwritten by the solution, and
+// the upper diagonals; the eliminated right-hand side takes the column's own place in u until the
+// solution does.  Levels are taken in whole chunks whose loads are issued together, then one by
+// one: a test per level inside a chunk (the level below N?) cost some 300 cycles a level.
+// Off: element offsets in a field (32-bit where they fit).
+template <typename R, int T, typename Off>
+__device__ __forceinline__ double roms_column(const Geo<R> &g, const int p, const int d, R *__restrict__ u,
+                                              RomsRhs<R> rs, R c0, R c1, R c2, const R *__restrict__ Hz,
                                               const R *__restrict__ Akv, const R *__restrict__ z_r,
-                                              const R *__restrict__ W, double avg, R on, R dt,
-                                              R lamdt) {
-    const long s2 = g.s2;
+                                              const R *__restrict__ W, double avg, R on, R dt, R lamdt,
+                                              R *__restrict__ col) {
+    const Off s2 = (Off)g.s2;
     const int N = g.N;
-    // the eliminated main and upper diagonals and right-hand side per level; the viscous
-    // coefficients FC, the vertical fluxes and the layer thicknesses are formed level by level
-    // (those of the level below carried in registers) and the thicknesses formed again for the
-    // sums: the same operations, in the same order, as storing them
-    R bc[kRomsMaxN], up[kRomsMaxN], rhs[kRomsMaxN];
-    const R pmU = R(0.5) * (g.pm[p] + g.pm[p - d]);
-    const R pnU = R(0.5) * (g.pn[p] + g.pn[p - d]);
-    const R fac = dt * (pmU * pnU);
+    const R pmU = rmul(R(0.5), g.pm[p] + g.pm[p - d]);
+    const R pnU = rmul(R(0.5), g.pn[p] + g.pn[p - d]);
+    const R fac = rmul(dt, rmul(pmU, pnU));
     auto wplus = [](R w) { return w > R(0) ? w : R(0); };
     auto wminus = [](R w) { return w < R(0) ? w : R(0); };
     R fcm = R(0), wk = R(0);   // FC of the level below, the flux through this level's bottom
-    // the levels' loads (independent of the elimination) issued kC levels at a time: one
-    // exposed load latency per chunk instead of per level (basin4: 4.70 ms with one level at a
-    // time, 3.58 with 4, 4.22 with 8 at 128 registers)
-    constexpr int kC = 4;
-    for (int k0 = 0; k0 < N; k0 += kC) {
-        R hz0[kC], hz1[kC], ak0[kC], ak1[kC], zr0[kC], zr1[kC], zq0[kC], zq1[kC], w0[kC], w1[kC],
-            q0[kC], q1[kC], q2[kC], uo[kC];
+    R pv = R(1), upp = R(0), xp = R(0);   // the level below's eliminated row (none: w = 0 / 1)
+    R zr = z_r[p], zq = z_r[p - d];       // z_r of the level in hand, both rho points
+    double H = 0.0;
+    R *bu = col;                          // the level's pivot, upper diagonal at bu[T]
+    Off o = (Off)p;
+    // elimination of a level: its FC and the flux through its top are given (0 at the surface)
+    auto eliminate = [&](R hza, R hzb, R fck, R wk1, R q0, R q1, R q2, R uo) {
+        const R hzu = rmul(R(0.5), hza + hzb);
+        R b = ((hzu - fck) - fcm) + (wplus(wk1) - wminus(wk));
+        const R upk = fck + wminus(wk1);
+        const R r = rfma(c2, q2, rfma(c0, q0, rmul(c1, q1)));
+        R x = rfma(hzu, uo, rmul(fac, r));
+        const R w = over_pivot(fcm - wplus(wk), pv);
+        b = rfma(-w, upp, b);
+        x = rfma(-w, xp, x);
+        pv = roms_pivot(b);
+        bu[0] = pv;
+        bu[T] = upk;
+        bu += 2 * T;
+        u[o] = x;
+        o += s2;
+        H = H + (double)hzu;
+        upp = upk;
+        xp = x;
+        fcm = fck;
+        wk = wk1;
+    };
+    auto levels = [&](auto n) {   // levels below the surface one
+        constexpr int C = decltype(n)::value;
+        R hz0[C], hz1[C], ak0[C], ak1[C], zr0[C], zq0[C], w0[C], w1[C], q0[C], q1[C], q2[C], uo[C];
+        Off l = o;
 #pragma unroll
-        for (int c = 0; c < kC; ++c) {
-            const int k = k0 + c < N ? k0 + c : N - 1;
-            const int kn = k + 1 < N ? k + 1 : N - 1;   // the next level (unused at the top)
-            const long o = (long)k * s2 + p, on_ = (long)kn * s2 + p;
-            hz0[c] = Hz[o];
-            hz1[c] = Hz[o - d];
-            ak0[c] = Akv[on_];
-            ak1[c] = Akv[on_ - d];
-            zr0[c] = z_r[on_];
-            zr1[c] = z_r[o];
-            zq0[c] = z_r[on_ - d];
-            zq1[c] = z_r[o - d];
-            w0[c] = W[on_];
-            w1[c] = W[on_ - d];
-            q0[c] = rs.r0[o];
-            q1[c] = rs.r1[o];
-            q2[c] = rs.r2[o];
-            uo[c] = u[o];
+        for (int c = 0; c < C; ++c, l += s2) {
+            const Off t = l + s2;
+            hz0[c] = Hz[l];
+            hz1[c] = Hz[l - d];
+            ak0[c] = Akv[t];
+            ak1[c] = Akv[t - d];
+            zr0[c] = z_r[t];
+            zq0[c] = z_r[t - d];
+            w0[c] = W[t];
+            w1[c] = W[t - d];
+            q0[c] = rs.r0[l];
+            q1[c] = rs.r1[l];
+            q2[c] = rs.r2[l];
+            uo[c] = u[l];
         }
 #pragma unroll
-        for (int c = 0; c < kC; ++c) {
-            const int k = k0 + c;
-            if (k >= N) break;
-            const R hzu = R(0.5) * (hz0[c] + hz1[c]);
-            R fck, wk1;
-            if (k < N - 1) {
-                const R ak = R(0.5) * (ak0[c] + ak1[c]);
-                const R dz = R(0.5) * ((zr0[c] - zr1[c]) + (zq0[c] - zq1[c]));
-                fck = ddiv(-lamdt * ak, dz);
-                wk1 = fac * (R(0.5) * (w0[c] + w1[c]));
-            } else {
-                fck = R(0);
-                wk1 = R(0);
-            }
-            const R fcm_k = k > 0 ? fcm : R(0);
-            R b = ((hzu - fck) - fcm_k) + (wplus(wk1) - wminus(wk));
-            up[k] = fck + wminus(wk1);
-            const R r = (c0 * q0[c] + c1 * q1[c]) + c2 * q2[c];
-            R x = hzu * uo[c] + fac * r;
-            if (k > 0) {
-                const R w = ddiv(fcm_k - wplus(wk), bc[k - 1]);
-                b = b - w * up[k - 1];
-                x = x - w * rhs[k - 1];
-            }
-            bc[k] = b;
-            rhs[k] = x;
-            fcm = fck;
-            wk = wk1;
+        for (int c = 0; c < C; ++c) {
+            const R ak = rmul(R(0.5), ak0[c] + ak1[c]);
+            const R dz = rmul(R(0.5), (zr0[c] - zr) + (zq0[c] - zq));
+            zr = zr0[c];
+            zq = zq0[c];
+            eliminate(hz0[c], hz1[c], roms_div(rmul(-lamdt, ak), dz), rmul(fac, rmul(R(0.5), w0[c] + w1[c])), q0[c],
+                      q1[c], q2[c], uo[c]);
         }
-    }
-    rhs[N - 1] = ddiv(rhs[N - 1], bc[N - 1]);          // x overwrites rhs
-    for (int k = N - 2; k >= 0; --k) rhs[k] = ddiv(rhs[k] - up[k] * rhs[k + 1], bc[k]);
-    double H = 0.0, Hu = 0.0;
-    constexpr int kS = 8;   // the thicknesses' loads kS levels at a time
-    for (int k0 = 0; k0 < N; k0 += kS) {
-        R ha[kS], hb[kS];
+    };
+    in_chunks<roms_col_chunk<R>()>(N - 1, levels);
+    eliminate(Hz[o], Hz[o - d], R(0), R(0), rs.r0[o], rs.r1[o], rs.r2[o], u[o]);
+    // back substitution
+    R x = over_pivot(xp, pv);
+    bu -= 2 * T;
+    bu[0] = x;
+    o -= s2;
+    auto back = [&](auto n) {
+        constexpr int C = decltype(n)::value;
+        R q[C], pk[C], uk[C];
 #pragma unroll
-        for (int c = 0; c < kS; ++c) {
-            const long o = (long)(k0 + c < N ? k0 + c : N - 1) * s2 + p;
-            ha[c] = Hz[o];
-            hb[c] = Hz[o - d];
+        for (int c = 0; c < C; ++c) {
+            o -= s2;
+            q[c] = u[o];
+            pk[c] = bu[-2 * T * (c + 1)];
+            uk[c] = bu[-2 * T * (c + 1) + T];
         }
 #pragma unroll
-        for (int c = 0; c < kS; ++c) {
-            if (k0 + c >= N) break;
-            const R hzu = R(0.5) * (ha[c] + hb[c]);
-            H = H + (double)hzu;
-            Hu = Hu + (double)hzu * (double)rhs[k0 + c];
+        for (int c = 0; c < C; ++c) {
+            bu -= 2 * T;
+            x = over_pivot(rfma(-uk[c], x, q[c]), pk[c]);
+            bu[0] = x;
         }
-    }
+    };
+    in_chunks<8>(N - 1, back);
+    double Hu = 0.0;
+    o = (Off)p;
+#pragma unroll 8
+    for (int k = 0; k < N; ++k, o += s2)
+        Hu = rsum<R>(Hu, (double)rmul(R(0.5), Hz[o] + Hz[o - d]), (double)col[k * (2 * T)]);
     const double target = avg / (double)on;
     const double udiff = (Hu - target) / H;
-    for (int k = 0; k < N; ++k) u[(long)k * s2 + p] = (R)((double)rhs[k] - udiff);
+    o = (Off)p;
+#pragma unroll 8
+    for (int k = 0; k < N; ++k, o += s2) u[o] = (R)((double)col[k * (2 * T)] - udiff);
     return target / H;
 }
 
-// The ROMS-form step3d_uv over the interior faces (U: j = 1..J-2, i = 2..I-2; V: j = 2..J-2,
-// i = 1..I-2), one thread per face column (a rho point's west U column or its south V
-// column; ensembles: both, one after the other), and the barotropic restart: ubar, vbar in
-// slots n and scratch = the new depth-mean velocities at those faces, 0 elsewhere.
-// t < s2: the U column (west face) of rho point t; s2 <= t < 2 s2: the V column (south face)
-// of rho point t - s2.
+// Threads per block of the column solve: 2 N values of shared memory per thread.
 template <typename R>
+constexpr int roms_col_threads() { return sizeof(R) == 4 ? 128 : 64; }
+
+// The ROMS-form step3d_uv over the interior faces (U: j = 1..J-2, i = 2..I-2; V: j = 2..J-2,
+// i = 1..I-2), one thread per face column: the U column (west face) or the V column (south face,
+// vcol) of rho point p; and the barotropic restart: ubar, vbar in slots n and scratch = the new
+// depth-mean velocities at those faces, 0 elsewhere.
+template <typename R, int T, typename Off>
 __device__ __forceinline__ void roms_step3d_at(const Geo<R> &g, R *__restrict__ u,
                                                R *__restrict__ v, RomsRhs<R> ru, RomsRhs<R> rv,
                                                R c0, R c1, R c2, R *__restrict__ ubar_n,
@@ -718,22 +766,20 @@ __device__ __forceinline__ void roms_step3d_at(const Geo<R> &g, R *__restrict__ 
                                                const R *__restrict__ W,
                                                const double *__restrict__ DU,
                                                const double *__restrict__ DV, R dt, R lamdt,
-                                               const long t) {
-    if (t >= 2 * g.s2) return;
-    const bool vcol = t >= g.s2;
-    const long p = vcol ? t - g.s2 : t;
-    const int j = fdiv((int)p, g.dI), i = (int)p - j * g.I;
+                                               const long t, const bool vcol, R *col) {
+    if (t >= g.s2) return;
+    const int p = (int)t, j = fdiv(p, g.dI), i = p - j * g.I;
     R bar = R(0);
     if (!vcol) {
         if (i >= 2 && i <= g.I - 2 && j >= 1 && j <= g.J - 2)
-            bar = (R)roms_column(g, p, 1, u, ru, c0, c1, c2, Hz, Akv, z_r, W, DU[p], g.on_u[p], dt,
-                                 lamdt);
+            bar = (R)roms_column<R, T, Off>(g, p, 1, u, ru, c0, c1, c2, Hz, Akv, z_r, W, DU[p], g.on_u[p], dt,
+                                       lamdt, col);
         ubar_n[p] = bar;
         ubar_s[p] = bar;
     } else {
         if (j >= 2 && j <= g.J - 2 && i >= 1 && i <= g.I - 2)
-            bar = (R)roms_column(g, p, g.I, v, rv, c0, c1, c2, Hz, Akv, z_r, W, DV[p], g.om_v[p],
-                                 dt, lamdt);
+            bar = (R)roms_column<R, T, Off>(g, p, g.I, v, rv, c0, c1, c2, Hz, Akv, z_r, W, DV[p], g.om_v[p],
+                                       dt, lamdt, col);
         vbar_n[p] = bar;
         vbar_s[p] = bar;
     }
@@ -881,32 +927,35 @@ __global__ void __launch_bounds__(256) kb_roms_stress3d(const Member<R> *mt, con
     roms_stress3d_at(m.g, u + m.o3, v + m.o3, ru + m.o3, rv + m.o3, sustr + m.o2, svstr + m.o2,
                      rdrag2, m.p);
 }
-template <typename R>
-__global__ void __launch_bounds__(128) k_roms_step3d(Geo<R> g, R *u, R *v, RomsRhs<R> ru,
-                                                     RomsRhs<R> rv, R c0, R c1, R c2, R *ubar_n,
-                                                     R *vbar_n, R *ubar_s, R *vbar_s, const R *Hz,
-                                                     const R *Akv, const R *z_r, const R *W,
-                                                     const double *DU, const double *DV, R dt,
-                                                     R lamdt) {
-    roms_step3d_at(g, u, v, ru, rv, c0, c1, c2, ubar_n, vbar_n, ubar_s, vbar_s, Hz, Akv, z_r, W,
-                   DU, DV, dt, lamdt, tid_flat());
+// A point block's U columns and its V columns are consecutive blocks: Hz, Akv, z_r and W are then read
+// from DRAM once for both.
+template <typename R, typename Off>
+__global__ void __launch_bounds__(roms_col_threads<R>(), 3) k_roms_step3d(
+    Geo<R> g, R *u, R *v, RomsRhs<R> ru, RomsRhs<R> rv, R c0, R c1, R c2, R *ubar_n, R *vbar_n, R *ubar_s,
+    R *vbar_s, const R *Hz, const R *Akv, const R *z_r, const R *W, const double *DU, const double *DV, R dt,
+    R lamdt) {
+    constexpr int T = roms_col_threads<R>();
+    extern __shared__ __align__(16) unsigned char col_smem[];
+    roms_step3d_at<R, T, Off>(g, u, v, ru, rv, c0, c1, c2, ubar_n, vbar_n, ubar_s, vbar_s, Hz, Akv, z_r, W, DU, DV,
+                         dt, lamdt, (long)(blockIdx.x >> 1) * T + threadIdx.x, blockIdx.x & 1,
+                         reinterpret_cast<R *>(col_smem) + threadIdx.x);
 }
-template <typename R>
-__global__ void __launch_bounds__(128) kb_roms_step3d(const Member<R> *mt, const int2 *bm, R *u,
-                                                      R *v, RomsRhs<R> ru, RomsRhs<R> rv, R c0,
-                                                      R c1, R c2, R *ubar_n, R *vbar_n,
-                                                      R *ubar_s, R *vbar_s, const R *Hz,
-                                                      const R *Akv, const R *z_r, const R *W,
-                                                      const double *DU, const double *DV, R dt,
-                                                      R lamdt) {
-    const MemberAt<R> m = member_at(mt, bm, 128);
-    const long o3 = m.o3, o2 = m.o2;
+template <typename R, typename Off>
+__global__ void __launch_bounds__(roms_col_threads<R>(), 3) kb_roms_step3d(
+    const Member<R> *mt, const int2 *bm, R *u, R *v, RomsRhs<R> ru, RomsRhs<R> rv, R c0, R c1, R c2, R *ubar_n,
+    R *vbar_n, R *ubar_s, R *vbar_s, const R *Hz, const R *Akv, const R *z_r, const R *W, const double *DU,
+    const double *DV, R dt, R lamdt) {
+    constexpr int T = roms_col_threads<R>(), kPart = 128 / T;   // blocks of T columns in a block of the map
+    extern __shared__ __align__(16) unsigned char col_smem[];
+    const int2 mb = bm[blockIdx.x / (2 * kPart)];
+    const Member<R> &M = mt[mb.x];
+    const int part = (int)(blockIdx.x >> 1) % kPart;
+    const long o3 = M.off3, o2 = M.off2;
     const RomsRhs<R> a{ru.r0 + o3, ru.r1 + o3, ru.r2 + o3}, b{rv.r0 + o3, rv.r1 + o3, rv.r2 + o3};
-    if (m.p >= m.g.s2) return;
-    for (int col = 0; col < 2; ++col)   // the point's U column, then its V column
-        roms_step3d_at(m.g, u + o3, v + o3, a, b, c0, c1, c2, ubar_n + o2, vbar_n + o2,
-                       ubar_s + o2, vbar_s + o2, Hz + m.oN, Akv + o3, z_r + m.oN, W + o3,
-                       DU + o2, DV + o2, dt, lamdt, m.p + col * m.g.s2);
+    roms_step3d_at<R, T, Off>(M.g, u + o3, v + o3, a, b, c0, c1, c2, ubar_n + o2, vbar_n + o2, ubar_s + o2,
+                         vbar_s + o2, Hz + M.offN, Akv + o3, z_r + M.offN, W + o3, DU + o2, DV + o2, dt, lamdt,
+                         (long)mb.y * 128 + part * T + threadIdx.x, blockIdx.x & 1,
+                         reinterpret_cast<R *>(col_smem) + threadIdx.x);
 }
 template <typename R>
 __global__ void __launch_bounds__(256) k_roms_walls3d(Geo<R> g, R *u, R *v) {
@@ -971,16 +1020,32 @@ cudaError_t Ops<R>::roms_step3d(const sf_ctx *c, R *u, R *v, const R *const *ru,
                                 const double *DU, const double *DV, double dt, double lamdt,
                                 cudaStream_t s) {
     const RomsRhs<R> a{ru[0], ru[1], ru[2]}, b{rv[0], rv[1], rv[2]};
+    constexpr int T = roms_col_threads<R>();
+    static bool done[64] = {};   // the raised shared-memory limit, once on each device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+        const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        const int most = 2 * kRomsMaxN * T * (int)sizeof(R);
+        for (auto k : {k_roms_step3d<R, int>, k_roms_step3d<R, long>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, most);
+        for (auto k : {kb_roms_step3d<R, int>, kb_roms_step3d<R, long>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, most);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) done[dev] = true;
+    }
+    const int N = c->nmem > 1 ? c->maxN : c->N, smem = 2 * N * T * (int)sizeof(R);
+    // 32-bit offsets within a member's field: (N + 2) levels of at most the pool's points
+    const bool fits = (long)(N + 2) * c->s2 < (1L << 31);
     if (c->nmem > 1)
-        kb_roms_step3d<R><<<c->nbm_128, 128, 0, s>>>(mt<R>(c), c->bm_128, u, v, a, b, (R)coef[0],
-                                                      (R)coef[1], (R)coef[2], ubar_n, vbar_n,
-                                                      ubar_s, vbar_s, Hz, Akv, z_r, W, DU, DV,
-                                                      (R)dt, (R)lamdt);
+        (fits ? kb_roms_step3d<R, int> : kb_roms_step3d<R, long>)<<<2 * (128 / T) * c->nbm_128, T, smem, s>>>(
+            mt<R>(c), c->bm_128, u, v, a, b, (R)coef[0], (R)coef[1], (R)coef[2], ubar_n, vbar_n, ubar_s, vbar_s,
+            Hz, Akv, z_r, W, DU, DV, (R)dt, (R)lamdt);
     else
-        k_roms_step3d<R><<<blocks_for(2 * c->s2, 128), 128, 0, s>>>(geo(c), u, v, a, b, (R)coef[0],
-                                                                  (R)coef[1], (R)coef[2], ubar_n,
-                                                                  vbar_n, ubar_s, vbar_s, Hz, Akv,
-                                                                  z_r, W, DU, DV, (R)dt, (R)lamdt);
+        (fits ? k_roms_step3d<R, int> : k_roms_step3d<R, long>)<<<2 * blocks_for(c->s2, T), T, smem, s>>>(
+            geo(c), u, v, a, b, (R)coef[0], (R)coef[1], (R)coef[2], ubar_n, vbar_n, ubar_s, vbar_s, Hz, Akv, z_r,
+            W, DU, DV, (R)dt, (R)lamdt);
     return cudaGetLastError();
 }
 template <typename R>
