@@ -29,166 +29,276 @@ __device__ __forceinline__ R qpow(R a, R b) { return pow(a, b); }
 template <>
 __device__ __forceinline__ float qpow<float>(float a, float b) { return powf(a, b); }
 
+// x^e for the models' exponents.  A multiple of 1/2 up to 8 (every exponent of k-epsilon and k-omega, the
+// exponent m of the generic model) is products and one square root; others take pow.  The test is
+// the same for every thread.
+struct GlsExp {
+    int h;       // 2 e, or kGlsPow
+    double e;
+};
+constexpr int kGlsPow = 1 << 20;
+inline GlsExp gls_exp(double e) {
+    GlsExp x;
+    x.e = e;
+    x.h = e * 2.0 == floor(e * 2.0) && fabs(e) <= 8.0 ? (int)(2.0 * e) : kGlsPow;
+    return x;
+}
 template <typename R>
-__global__ void __launch_bounds__(128) k_gls_corrector(
-    Geo<R> g, sf_gls_params P, R dt, const R *__restrict__ u, const R *__restrict__ v,
-    const R *__restrict__ z_r, const R *__restrict__ Hz, const R *__restrict__ bvf,
-    const R *__restrict__ sustr, const R *__restrict__ svstr, R *tke, R *gls, R *Akv, R *Akt,
-    R *Akk, R *Akp, R *Lscale, const R *__restrict__ tkn0, const R *__restrict__ gln0,
-    const uint8_t *__restrict__ sel, const int *__restrict__ list, const int *__restrict__ count) {
+__device__ __forceinline__ R gls_pow(R x, GlsExp e) {
+    if (e.h == kGlsPow) return qpow(x, (R)e.e);
+    const int a = e.h < 0 ? -e.h : e.h, n = a >> 1;
+    R r = a & 1 ? sqrt(x) : R(1);
+    if (n) {
+        R q = x;
+        if (n & 1) r *= q;
+        if (n > 1) {
+            q *= q;
+            if (n & 2) r *= q;
+            if (n > 3) {
+                q *= q;
+                if (n & 4) r *= q;
+                if (n & 8) r *= q * q;
+            }
+        }
+    }
+    return e.h < 0 ? R(1) / r : r;
+}
+
+// The model's constants, evaluated once on the host in FP64 (a column evaluated a dozen powers of
+// them), and its exponents.
+template <typename R>
+struct GlsConst {
+    R dt, Kmin, Pmin, Akv_bak, Akt_bak, Akk_bak, Akp_bak, c1, c2, c3m, c3p, sigk, sigp, ogls_sigp, rdrag2;
+    R cmu0, cmu_fac1, cmu_fac2, cmu_fac3, cmu0p, Zos, Zob, glsN, gls0, fluxt, fluxb;
+    GlsExp m, n, in, mi, n1;   // m, n, 1/n, -1/n, n - 1
+};
+template <typename R>
+GlsConst<R> gls_const(const sf_gls_params &P, double dt) {
+    GlsConst<R> G;
+    const double Zos = fmax(P.Zos, 1.0e-4), Zob = fmax(P.Zob, 1.0e-4), cp = pow(P.cmu0, P.p);
+    G.dt = (R)dt;
+    G.Kmin = (R)P.Kmin;
+    G.Pmin = (R)P.Pmin;
+    G.Akv_bak = (R)P.Akv_bak;
+    G.Akt_bak = (R)P.Akt_bak;
+    G.Akk_bak = (R)P.Akk_bak;
+    G.Akp_bak = (R)P.Akp_bak;
+    G.c1 = (R)P.c1;
+    G.c2 = (R)P.c2;
+    G.c3m = (R)P.c3m;
+    G.c3p = (R)P.c3p;
+    G.sigk = (R)P.sigk;
+    G.sigp = (R)P.sigp;
+    G.ogls_sigp = (R)(1.0 / P.sigp);
+    G.rdrag2 = (R)P.rdrag2;
+    G.cmu0 = (R)P.cmu0;
+    G.cmu_fac1 = (R)pow(P.cmu0, -P.p / P.n);
+    G.cmu_fac2 = (R)pow(P.cmu0, 3.0 + P.p / P.n);
+    G.cmu_fac3 = (R)(1.0 / (P.cmu0 * P.cmu0));
+    G.cmu0p = (R)cp;
+    G.Zos = (R)Zos;
+    G.Zob = (R)Zob;
+    G.glsN = (R)(cp * pow(kVonKar * Zos, P.n));
+    G.gls0 = (R)(cp * pow(kVonKar * Zob, P.n));
+    G.fluxt = (R)(dt * cp * P.n * pow(kVonKar, P.n) * 0.5);
+    G.fluxb = (R)(dt * cp * P.n * pow(kVonKar, P.n) * 0.5);
+    G.m = gls_exp(P.m);
+    G.n = gls_exp(P.n);
+    G.in = gls_exp(1.0 / P.n);
+    G.mi = gls_exp(-1.0 / P.n);
+    G.n1 = gls_exp(P.n - 1.0);
+    return G;
+}
+
+// One thread per column.  Bound: 76 bytes a point and level in FP32 (12 fields read, 7 written: 0.31 ms for
+// 1026 x 514 x 50 at the copy bandwidth) and its instructions: the column used to take eight pow a
+// level and seven local arrays (1.98 ms; FP64 generic model, 514 x 258 x 32: 0.84 ms).  Three passes:
+//   down  production, dissipation and the elimination of both systems.  The gls surface flux needs
+//         the solved tke: it enters the top row linearly, so a second right-hand side b (1 in the top
+//         row, 0 below) is eliminated beside the first and scaled later.
+//   up    tke.
+//   up    gls and the coefficients.
+// What a pass leaves for the next lies in the column's own outputs, whose old values have been used by
+// then: CF and the eliminated tke in Akv and Akt, CF and the two right-hand sides of gls in Akk, gls
+// and Akp.  Powers: with psi = cmu0^p k^m l^n, psi / k^m depends on l alone, so each of the dissipation,
+// the length scale and the limited psi takes one power of l; the upper limit on l that stratification
+// sets (a limit on psi in the reference's text) is compared as a length, without one.
+// Blocks per SM: the levels are a chain of divisions and roots, so warps hide the latency, not loads in
+// flight (levels in chunks of 4 at 128 registers: 0.97 and 0.41 ms for the two cases above; one at a
+// time with 10 blocks at 48 registers in FP32, 7 at 72 in FP64: 0.76 and 0.31; 12 blocks 0.88).
+template <typename R>
+constexpr int gls_blocks() { return sizeof(R) == 4 ? 10 : 7; }
+template <typename R, typename Off>
+__global__ void __launch_bounds__(128, gls_blocks<R>()) k_gls_corrector(
+    Geo<R> g, const GlsConst<R> G, const R *__restrict__ u, const R *__restrict__ v, const R *__restrict__ z_r,
+    const R *__restrict__ Hz, const R *__restrict__ bvf, const R *__restrict__ sustr,
+    const R *__restrict__ svstr, R *tke, R *gls, R *Akv, R *Akt, R *Akk, R *Akp, R *Lscale,
+    const R *__restrict__ tkn0, const R *__restrict__ gln0, const uint8_t *__restrict__ sel,
+    const int *__restrict__ list, const int *__restrict__ count) {
     int pi = (int)tid_flat();
     if (list) {                    // a compacted list of columns: thread t takes list[t]
         if (pi >= *count) return;
         pi = list[pi];
     }
     if (pi >= g.s2) return;
-    const int i = pi % g.I, j = pi / g.I;
+    const int j = fdiv(pi, g.dI), i = pi - j * g.I;
     if (!rint_(i, j, g.I, g.J)) return;
     if (sel && !sel[pi]) return;   // column not selected: left as it is
-    const long p = pi, I = g.I, s2 = g.s2;
-    const int N = g.N;
-    R FCK[kNMax + 1], FCP[kNMax + 1], BCK[kNMax + 1], BCP[kNMax + 1], tk[kNMax + 1], gl[kNMax + 1],
-        CF[kNMax + 1];
-#define AT(X, k, q) ((X)[(long)(k) * s2 + (q)])
-    const R pp = (R)P.p, mm = (R)P.m, nn = (R)P.n, cmu0 = (R)P.cmu0;
-    const R L_sft = (R)kVonKar, ogls_sigp = R(1) / (R)P.sigp;
-    const R cmu_fac1 = qpow(cmu0, -pp / nn), cmu_fac2 = qpow(cmu0, R(3) + pp / nn);
-    const R cmu_fac3 = R(1) / qpow(cmu0, R(2));
-    const R gls_fac2 = qpow(cmu0, pp) * nn * qpow((R)kVonKar, nn), gls_fac3 = qpow(cmu0, pp) * nn;
-    const R gls_fac4 = qpow(cmu0, pp), gls_fac5 = qpow(R(0.56), R(0.5) * nn) * qpow(cmu0, pp);
-    const R gls_exp1 = R(1) / nn, tke_exp1 = mm / nn, tke_exp2 = R(0.5) + mm / nn;
-    const R tke_exp4 = mm + R(0.5) * nn;
-    const R Kmin = (R)P.Kmin, Pmin = (R)P.Pmin, eps = (R)kGlsEps;
-    const R Zos_eff = (R)fmax(P.Zos, 1.0e-4), Zob_min = (R)fmax(P.Zob, 1.0e-4);
-    const R Akv_bak = (R)P.Akv_bak, Akt_bak = (R)P.Akt_bak, Akk_bak = (R)P.Akk_bak,
-            Akp_bak = (R)P.Akp_bak;
+    const Off p = (Off)pi, s2 = (Off)g.s2;
+    const int I = g.I, N = g.N;
+    const R dt = G.dt, Kmin = G.Kmin, Pmin = G.Pmin, eps = (R)kGlsEps;
 
-    // vertical mixing of the turbulent fields (:401-415)
-    FCK[1] = FCK[N] = FCP[1] = FCP[N] = R(0);
-    for (int k = 2; k < N; ++k) {
-        const R hz = AT(Hz, k - 1, p);
-        FCK[k] = (R(-0.5) * dt) * (AT(Akk, k, p) + AT(Akk, k - 1, p)) / hz;
-        FCP[k] = (R(-0.5) * dt) * (AT(Akp, k, p) + AT(Akp, k - 1, p)) / hz;
-    }
-    // production and dissipation (:397-516)
-    for (int k = 1; k < N; ++k) {
-        const R cff = R(0.5) / (AT(z_r, k, p) - AT(z_r, k - 1, p));
-        const R du = (AT(u, k, p) - AT(u, k - 1, p)) + (AT(u, k, p + 1) - AT(u, k - 1, p + 1));
-        const R dv = (AT(v, k, p) - AT(v, k - 1, p)) + (AT(v, k, p + I) - AT(v, k - 1, p + I));
+    // --- down: levels N-1 .. 1
+    Off o = p + (Off)(N - 1) * s2;   // W level k, rho level k + 1 in Fortran numbering
+    R ut = u[o] , ute = u[o + 1], vt = v[o], vtn = v[o + I], zt = z_r[o], hzt = Hz[o];
+    R akk = Akk[o], akp = Akp[o];
+    const R akpN = Akp[o + s2] + akp, AkpB = Akp[p] + Akp[p + s2];
+    R fk1 = R(0), fp1 = R(0);               // FCK, FCP of the level above
+    R cfk = R(0), tk = R(0), cfp = R(0), ga = R(0), gb = R(0), cffp = R(0);   // its eliminated rows
+    R top = R(1);
+    for (int k = N - 1; k >= 1; --k) {
+        const Off b = o - s2;
+        const R ub = u[b], ube = u[b + 1], vb = v[b], vbn = v[b + I], zb = z_r[b], hb = Hz[b];
+        const R kk = Akk[b], kp = Akp[b], av = Akv[o], at = Akt[o], tko = tke[o], glo = gls[o], strat2 = bvf[o];
+        // vertical mixing of the turbulent fields (:401-415), none through the lowest layer
+        const bool lowest = k == 1;
+        const R fk = lowest ? R(0) : (R(-0.5) * dt) * (akk + kk) / hb;
+        const R fp = lowest ? R(0) : (R(-0.5) * dt) * (akp + kp) / hb;
+        // production and dissipation (:397-516)
+        const R cff = R(0.5) / (zt - zb);
+        const R du = (ut - ub) + (ute - ube), dv = (vt - vb) + (vtn - vbn);
         const R sh2 = (cff * du) * (cff * du) + (cff * dv) * (cff * dv);
-        const R cffz = R(0.5) * (AT(Hz, k - 1, p) + AT(Hz, k, p));
-        const R tko = AT(tke, k, p), glo = AT(gls, k, p);
-        const R strat2 = AT(bvf, k, p);
-        const R c3 = strat2 > R(0) ? (R)P.c3m : (R)P.c3p;
-        const R dAkt = AT(Akt, k, p) - Akt_bak, dAkv = AT(Akv, k, p) - Akv_bak;
-        R Kprod = sh2 * dAkv - strat2 * dAkt;
-        R Pprod = (R)P.c1 * sh2 * dAkv - c3 * strat2 * dAkt;
-        R cff1 = R(1), cff2 = R(1);
+        const R cffz = R(0.5) * (hb + hzt);
+        const R c3 = strat2 > R(0) ? G.c3m : G.c3p;
+        const R dAkt = at - G.Akt_bak, dAkv = av - G.Akv_bak, buo = strat2 * dAkt;
+        R Kprod = sh2 * dAkv - buo;
+        R Pprod = G.c1 * sh2 * dAkv - c3 * buo;
+        R sk = R(0), sp = R(0);   // the buoyancy terms taken implicitly
         if (Kprod < R(0)) {
-            Kprod = Kprod + strat2 * dAkt;
-            cff1 = R(0);
+            Kprod = Kprod + buo;
+            sk = buo;
         }
         if (Pprod < R(0)) {
-            Pprod = Pprod + c3 * strat2 * dAkt;
-            cff2 = R(0);
+            Pprod = Pprod + c3 * buo;
+            sp = c3 * buo;
         }
         // the new level starts from tke/gls(nnew) after advection when given, else from
         // Hz_w * tke/gls(nstp) (the predictor's start without the advective terms)
-        const R tst = tkn0 ? AT(tkn0, k, p) : cffz * tko;
-        const R gst = gln0 ? AT(gln0, k, p) : cffz * glo;
-        tk[k] = tst + dt * cffz * Kprod;
-        gl[k] = gst + dt * cffz * Pprod * glo / fmax(tko, Kmin);
-        const R diss = qpow(glo, -gls_exp1) * cmu_fac2 * qpow(tko, tke_exp2);
-        BCK[k] = cffz * (R(1) + dt * diss + dt * (R(1) - cff1) * strat2 * dAkt / tko) - FCK[k] -
-                 (k + 1 <= N ? FCK[k + 1] : R(0));
-        BCP[k] = cffz * (R(1) + dt * (R)P.c2 * diss + dt * (R(1) - cff2) * c3 * strat2 * dAkt / tko) -
-                 FCP[k] - (k + 1 <= N ? FCP[k + 1] : R(0));
+        const R tr = (tkn0 ? tkn0[o] : cffz * tko) + dt * cffz * Kprod;
+        const R gr = (gln0 ? gln0[o] : cffz * glo) + dt * cffz * Pprod * glo / fmax(tko, Kmin);
+        const R diss = G.cmu_fac2 * gls_pow(glo / gls_pow(tko, G.m), G.mi) * sqrt(tko);
+        const R bck = cffz * (R(1) + dt * diss + dt * sk / tko) - fk - fk1;
+        const R bcp = cffz * (R(1) + dt * G.c2 * diss + dt * sp / tko) - fp - fp1;
+        // tke (:571-604) and gls (:608-656) eliminated
+        const R ck = R(1) / (bck - cfk * fk1);
+        cfk = ck * fk;
+        tk = ck * (tr - fk1 * tk);
+        cffp = R(1) / (bcp - cfp * fp1);
+        cfp = cffp * fp;
+        ga = cffp * (gr - fp1 * ga);
+        gb = cffp * (top - fp1 * gb);
+        top = R(0);
+        Akv[o] = cfk;
+        Akt[o] = tk;
+        Akk[o] = cfp;
+        gls[o] = ga;
+        Akp[o] = gb;
+        fk1 = fk;
+        fp1 = fp;
+        akk = kk;
+        akp = kp;
+        ut = ub;
+        ute = ube;
+        vt = vb;
+        vtn = vbn;
+        zt = zb;
+        hzt = hb;
+        o = b;
     }
     // surface and bottom conditions (:526-564); bottom stress on the bottom-level velocity
-    auto bustr = [&](long q) {
-        const R va = R(0.25) * (AT(v, 0, q) + AT(v, 0, q + I) + AT(v, 0, q - 1) + AT(v, 0, q - 1 + I));
-        return (R)P.rdrag2 * AT(u, 0, q) * sqrt(AT(u, 0, q) * AT(u, 0, q) + va * va);
+    auto bustr = [&](Off q) {
+        const R va = R(0.25) * (v[q] + v[q + I] + v[q - 1] + v[q - 1 + I]);
+        return G.rdrag2 * u[q] * sqrt(u[q] * u[q] + va * va);
     };
-    auto bvstr = [&](long q) {
-        const R ua = R(0.25) * (AT(u, 0, q) + AT(u, 0, q + 1) + AT(u, 0, q - I) + AT(u, 0, q + 1 - I));
-        return (R)P.rdrag2 * AT(v, 0, q) * sqrt(ua * ua + AT(v, 0, q) * AT(v, 0, q));
+    auto bvstr = [&](Off q) {
+        const R ua = R(0.25) * (u[q] + u[q + 1] + u[q - I] + u[q + 1 - I]);
+        return G.rdrag2 * v[q] * sqrt(ua * ua + v[q] * v[q]);
     };
     const R su = sustr[p] + sustr[p + 1], sv = svstr[p] + svstr[p + I];
     const R bu = bustr(p) + bustr(p + 1), bv = bvstr(p) + bvstr(p + I);
-    tk[N] = fmax(cmu_fac3 * R(0.5) * sqrt(su * su + sv * sv), Kmin);
-    tk[0] = fmax(cmu_fac3 * R(0.5) * sqrt(bu * bu + bv * bv), Kmin);
-    gl[N] = fmax(qpow(cmu0, pp) * qpow(tk[N], mm) * qpow(L_sft * Zos_eff, nn), Pmin);
-    gl[0] = fmax(gls_fac4 * qpow((R)kVonKar * Zob_min, nn) * qpow(tk[0], mm), Pmin);
-    // tke (:571-604)
-    R cff = R(1) / BCK[N - 1];
-    CF[N - 1] = cff * FCK[N - 1];
-    tk[N - 1] = cff * tk[N - 1];
-    for (int k = N - 2; k >= 1; --k) {
-        cff = R(1) / (BCK[k] - CF[k + 1] * FCK[k + 1]);
-        CF[k] = cff * FCK[k];
-        tk[k] = cff * (tk[k] - FCK[k + 1] * tk[k + 1]);
-    }
-    tk[1] = fmax(tk[1], Kmin);
-    for (int k = 2; k < N; ++k) tk[k] = fmax(tk[k] - CF[k] * tk[k - 1], Kmin);
-    // gls (:608-656)
-    const R cffT = R(0.5) * (tk[N] + tk[N - 1]);
-    const R fluxt = dt * gls_fac3 * qpow(cffT, mm) * qpow(L_sft, nn) *
-                    qpow(Zos_eff + R(0.5) * AT(Hz, N - 1, p), nn - R(1)) * R(0.5) *
-                    (AT(Akp, N, p) + AT(Akp, N - 1, p));
-    const R cffB = R(0.5) * (tk[0] + tk[1]);
-    const R fluxb = dt * gls_fac2 * qpow(cffB, mm) * qpow(R(0.5) * AT(Hz, 0, p) + Zob_min, nn - R(1)) *
-                    R(0.5) * (AT(Akp, 0, p) + AT(Akp, 1, p));
-    cff = R(1) / BCP[N - 1];
-    CF[N - 1] = cff * FCP[N - 1];
-    gl[N - 1] = cff * (gl[N - 1] - fluxt);
-    for (int k = N - 2; k >= 1; --k) {
-        cff = R(1) / (BCP[k] - CF[k + 1] * FCP[k + 1]);
-        CF[k] = cff * FCP[k];
-        gl[k] = cff * (gl[k] - FCP[k + 1] * gl[k + 1]);
-    }
-    gl[1] = gl[1] - cff * fluxb;
-    for (int k = 2; k < N; ++k) gl[k] = gl[k] - CF[k] * gl[k - 1];
-    // mixing coefficients (:662-825); the old values of level k are read before it is written
+    const R tkN = fmax(G.cmu_fac3 * R(0.5) * sqrt(su * su + sv * sv), Kmin);
+    const R tk0 = fmax(G.cmu_fac3 * R(0.5) * sqrt(bu * bu + bv * bv), Kmin);
+    const R glN = fmax(gls_pow(tkN, G.m) * G.glsN, Pmin);
+    const R gl0 = fmax(G.gls0 * gls_pow(tk0, G.m), Pmin);
+    // --- up: tke
+    o = p + s2;
+    tk = fmax(tk, Kmin);
+    const R tk1 = tk;
+    Akt[o] = tk;
+    auto up = [&](auto nc) {
+        constexpr int C = decltype(nc)::value;
+        R a[C], f[C];
+        Off l = o;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            l += s2;
+            a[c] = Akt[l];
+            f[c] = Akv[l];
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            o += s2;
+            tk = fmax(a[c] - f[c] * tk, Kmin);
+            Akt[o] = tk;
+        }
+    };
+    in_chunks<4>(N - 2, up);
+    // fluxes of gls through the surface and the bottom (:608-630)
+    const R fluxt = G.fluxt * gls_pow(R(0.5) * (tkN + tk), G.m) *
+                    gls_pow(G.Zos + R(0.5) * Hz[p + (Off)(N - 1) * s2], G.n1) * akpN;
+    const R fluxb = G.fluxb * gls_pow(R(0.5) * (tk0 + tk1), G.m) * gls_pow(R(0.5) * Hz[p] + G.Zob, G.n1) * AkpB;
+    // --- up: gls and the mixing coefficients (:662-825); the old values of a level are read before they
+    // are written
     const R sqrt2 = sqrt(R(2));
+    R gl = cffp * fluxb;   // level 1 takes the bottom flux as the term below it
+    o = p + s2;
     for (int k = 1; k < N; ++k) {
-        const R b2 = AT(bvf, k, p);
-        const R tkn = fmax(tk[k], Kmin);
-        R gln = fmax(gl[k], Pmin);
-        const R lim = gls_fac5 * qpow(tkn, tke_exp4) * qpow(sqrt(fmax(R(0), b2)) + eps, -nn);
-        gln = nn >= R(0) ? fmin(gln, lim) : fmax(gln, lim);
-        const R Ls_unlmt = fmax(eps, qpow(gln, gls_exp1) * cmu_fac1 * qpow(tkn, -tke_exp1));
-        const R Ls_lmt = b2 > R(0) ? fmin(Ls_unlmt, sqrt(R(0.56) * tkn / (fmax(R(0), b2) + eps)))
-                                   : Ls_unlmt;
-        gln = fmax(qpow(cmu0, pp) * qpow(tkn, mm) * qpow(Ls_lmt, nn), Pmin);
-        R Gh = fmin((R)kGh0, -b2 * Ls_lmt * Ls_lmt / (R(2) * tkn));
+        const R a = gls[o], b = Akp[o], f = Akk[o], t = Akt[o], b2 = bvf[o], ls = Lscale[o], to = tke[o];
+        gl = (a - fluxt * b) - (k == 1 ? gl : f * gl);
+        const R b2p = fmax(R(0), b2);
+        const R tkn = fmax(t, Kmin), tm = gls_pow(tkn, G.m);
+        const R Ls_gl = G.cmu_fac1 * gls_pow(fmax(gl, Pmin) / tm, G.in);
+        const R Ls_unlmt = fmax(eps, fmin(Ls_gl, sqrt(R(0.56) * tkn) / (sqrt(b2p) + eps)));
+        const R Ls = b2 > R(0) ? fmin(Ls_unlmt, sqrt(R(0.56) * tkn / (b2p + eps))) : Ls_unlmt;
+        R Gh = fmin((R)kGh0, -b2 * Ls * Ls / (R(2) * tkn));
         Gh = fmin(Gh, Gh - (Gh - (R)kGhcri) * (Gh - (R)kGhcri) / (Gh + (R)kGh0 - R(2) * (R)kGhcri));
         Gh = fmax(Gh, (R)kGhmin);
         const R Sh = (R)kSh1 / (R(1) - (R)kSh2 * Gh);
         const R Sm = ((R)kSm3 + Sh * Gh * (R)kSm4) / (R(1) - (R)kSm2 * Gh);
-        const R ql = sqrt2 * R(0.5) * (Ls_lmt * sqrt(tkn) + AT(Lscale, k, p) * sqrt(AT(tke, k, p)));
-        AT(Akv, k, p) = Akv_bak + Sm * ql;
-        AT(Akt, k, p) = Akt_bak + Sh * ql;
-        AT(Akk, k, p) = Akk_bak + Sm * ql / (R)P.sigk;
-        AT(Akp, k, p) = Akp_bak + Sm * ql * ogls_sigp;
-        AT(Lscale, k, p) = Ls_lmt;
-        AT(tke, k, p) = tkn;
-        AT(gls, k, p) = gln;
+        const R ql = sqrt2 * R(0.5) * (Ls * sqrt(tkn) + ls * sqrt(to));
+        Akv[o] = G.Akv_bak + Sm * ql;
+        Akt[o] = G.Akt_bak + Sh * ql;
+        Akk[o] = G.Akk_bak + Sm * ql / G.sigk;
+        Akp[o] = G.Akp_bak + Sm * ql * G.ogls_sigp;
+        Lscale[o] = Ls;
+        tke[o] = tkn;
+        gls[o] = fmax(G.cmu0p * tm * gls_pow(Ls, G.n), Pmin);
+        o += s2;
     }
-    const R AvN = Akv_bak + L_sft * Zos_eff * cmu0 * sqrt(tk[N]);
-    const R Av0 = Akv_bak + (R)kVonKar * Zob_min * cmu0 * sqrt(tk[0]);
-    AT(Akv, N, p) = AvN;
-    AT(Akv, 0, p) = Av0;
-    AT(Akk, N, p) = Akk_bak + AvN / (R)P.sigk;
-    AT(Akk, 0, p) = Akk_bak + Av0 / (R)P.sigk;
-    AT(Akp, N, p) = Akp_bak + AvN * ogls_sigp;
-    AT(Akp, 0, p) = Akp_bak + Av0 / (R)P.sigp;
-    AT(Akt, N, p) = Akt_bak;
-    AT(Akt, 0, p) = Akt_bak;
-    AT(tke, N, p) = tk[N];
-    AT(tke, 0, p) = tk[0];
-    AT(gls, N, p) = gl[N];
-    AT(gls, 0, p) = gl[0];
-#undef AT
+    const R AvN = G.Akv_bak + (R)kVonKar * G.Zos * G.cmu0 * sqrt(tkN);
+    const R Av0 = G.Akv_bak + (R)kVonKar * G.Zob * G.cmu0 * sqrt(tk0);
+    Akv[o] = AvN;   // o is level N here
+    Akv[p] = Av0;
+    Akk[o] = G.Akk_bak + AvN / G.sigk;
+    Akk[p] = G.Akk_bak + Av0 / G.sigk;
+    Akp[o] = G.Akp_bak + AvN * G.ogls_sigp;
+    Akp[p] = G.Akp_bak + Av0 / G.sigp;
+    Akt[o] = G.Akt_bak;
+    Akt[p] = G.Akt_bak;
+    tke[o] = tkN;
+    tke[p] = tk0;
+    gls[o] = glN;
+    gls[p] = gl0;
 }
 
 

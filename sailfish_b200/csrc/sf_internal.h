@@ -216,6 +216,22 @@ inline cudaError_t launch_dep(const sf_ctx *c, void (*kern)(KArgs...), dim3 grid
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// f(C) for n levels in chunks of C, what is left in chunks of 4, 2 and 1: the levels of a chunk carry no
+// test against n.
+template <int C, typename F>
+__device__ __forceinline__ void in_chunks(int n, F f) {
+    for (; n >= C; n -= C) f(std::integral_constant<int, C>());
+    if (C > 4 && n >= 4) {
+        f(std::integral_constant<int, 4>());
+        n -= 4;
+    }
+    if (C > 2 && n >= 2) {
+        f(std::integral_constant<int, 2>());
+        n -= 2;
+    }
+    if (n >= 1) f(std::integral_constant<int, 1>());
+}
+
 // Levels the ROMS-form step3d_uv holds per column (sf_roms_step3d_uv rejects more).
 constexpr int kRomsMaxN = 64;
 

@@ -2806,8 +2806,9 @@ cudaError_t Ops<R>::gls_corrector(const sf_ctx *c, const sf_gls_params &P, doubl
                                   R *Akk, R *Akp, R *Lscale, const R *tkn0,
                                   const R *gln0, const uint8_t *sel, const int *list,
                                   const int *count, cudaStream_t s) {
-    k_gls_corrector<R><<<blocks_for(c->s2, 128), 128, 0, s>>>(
-        geo(c), P, (R)dt, u, v, z_r, Hz, bvf, sustr, svstr, tke, gls, Akv, Akt, Akk, Akp, Lscale,
+    const bool fits = (long)(c->N + 2) * c->s2 < (1L << 31);   // 32-bit element offsets
+    (fits ? k_gls_corrector<R, int> : k_gls_corrector<R, long>)<<<blocks_for(c->s2, 128), 128, 0, s>>>(
+        geo(c), gls_const<R>(P, dt), u, v, z_r, Hz, bvf, sustr, svstr, tke, gls, Akv, Akt, Akk, Akp, Lscale,
         tkn0, gln0, sel, list, count);
     return cudaGetLastError();
 }

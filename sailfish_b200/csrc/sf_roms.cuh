@@ -604,20 +604,6 @@ struct RomsRhs {
 // 0.59, 0.47, 0.45, 0.53 ms, 118 to 197 registers; FP64 4, 6, 8: 1.29, 1.27, 1.33).
 template <typename R>
 constexpr int roms_col_chunk() { return sizeof(R) == 4 ? 8 : 6; }
-// f(C) for n levels in chunks of C, what is left in chunks of 4, 2 and 1
-template <int C, typename F>
-__device__ __forceinline__ void in_chunks(int n, F f) {
-    for (; n >= C; n -= C) f(std::integral_constant<int, C>());
-    if (n >= 4) {
-        f(std::integral_constant<int, 4>());
-        n -= 4;
-    }
-    if (n >= 2) {
-        f(std::integral_constant<int, 2>());
-        n -= 2;
-    }
-    if (n >= 1) f(std::integral_constant<int, 1>());
-}
 // A pivot of the elimination as its divisions use it: in FP32 the reciprocal (a / b through
 // __fdividef is a times the hardware reciprocal of b, bit for bit in b's normal range, and every
 // pivot divides twice), in FP64 the pivot itself (IEEE division).
