@@ -137,9 +137,9 @@ struct sf_ctx {
     // by default: on basin4 the column solve took 2.08 ms with it against 1.65 ms with
     // per-element cp.async staging
     int use_bulk = 0;
-    // levels whose loads the fused flux/omega kernel issues together (sf_ctx_tune; basin4:
-    // 0.82, 0.77 and 1.16 ms with 4, 5 and 8: 80, 80 and 128 registers)
-    int mo_chunk = 5;
+    // levels whose loads the fused flux/omega kernel issues together (sf_ctx_tune; 2050 x 1026 x 50 in
+    // FP32: 0.74, 0.76 and 0.86 ms with 4, 5 and 8 at 3 blocks per SM)
+    int mo_chunk = 4;
     // fused predictor in its paired form (two nodes per thread) where the grid allows it: 1
     // with 16-row blocks, 2 with 8-row blocks (basin4 loop 4.27 and 4.18 ms), 0 scalar (4.49)
     int pred_pair = 2;
@@ -216,20 +216,25 @@ inline cudaError_t launch_dep(const sf_ctx *c, void (*kern)(KArgs...), dim3 grid
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// f(C) for n levels in chunks of C, what is left in chunks of 4, 2 and 1: the levels of a chunk carry no
-// test against n.
+// f(C) for n levels in chunks of C (at most 32), what is left in chunks of the powers of two below C: the
+// levels of a chunk carry no test against n.
 template <int C, typename F>
 __device__ __forceinline__ void in_chunks(int n, F f) {
     for (; n >= C; n -= C) f(std::integral_constant<int, C>());
-    if (C > 4 && n >= 4) {
-        f(std::integral_constant<int, 4>());
-        n -= 4;
-    }
-    if (C > 2 && n >= 2) {
-        f(std::integral_constant<int, 2>());
-        n -= 2;
-    }
-    if (n >= 1) f(std::integral_constant<int, 1>());
+    auto rest = [&](auto w) {
+        constexpr int P = decltype(w)::value;
+        if constexpr (P < C) {
+            if (n >= P) {
+                f(w);
+                n -= P;
+            }
+        }
+    };
+    rest(std::integral_constant<int, 16>());
+    rest(std::integral_constant<int, 8>());
+    rest(std::integral_constant<int, 4>());
+    rest(std::integral_constant<int, 2>());
+    rest(std::integral_constant<int, 1>());
 }
 
 // Levels the ROMS-form step3d_uv holds per column (sf_roms_step3d_uv rejects more).

@@ -1418,12 +1418,14 @@ __device__ __forceinline__ void maxflux_omega_body(
         if (C < 0 && !rc) {
             // omega alone: the four fluxes of a chunk of kO levels loaded together (basin4:
             // 0.45 ms with 16, 0.48 with 8, 0.66 one level at a time)
-            constexpr int kO = 16;
-            for (int K0 = 1; K0 < N; K0 += kO) {
+            long o0 = s2 + p;
+            int K0 = 1;
+            in_chunks<16>(N - 1, [&](auto n) {
+                constexpr int kO = decltype(n)::value;
                 R hu[kO], hv[kO], hE[kO], hN[kO];
 #pragma unroll
                 for (int c = 0; c < kO; ++c) {
-                    const long o = (long)(K0 + c < N ? K0 + c : N - 1) * s2 + p;
+                    const long o = o0 + c * s2;
                     hu[c] = Huon[o];
                     hv[c] = Hvom[o];
                     hE[c] = Huon[o + 1];
@@ -1431,27 +1433,25 @@ __device__ __forceinline__ void maxflux_omega_body(
                 }
 #pragma unroll
                 for (int c = 0; c < kO; ++c) {
-                    if (K0 + c < N) {
-                        Wk = Wk - ((hE[c] - hu[c]) + (hN[c] - hv[c]));
-                        Wc(K0 + c) = Wk;
-                    }
+                    Wk = Wk - ((hE[c] - hu[c]) + (hN[c] - hv[c]));
+                    Wc(K0 + c) = Wk;
                 }
-            }
+                o0 += kO * s2;
+                K0 += kO;
+            });
         } else if (C > 0 && fu && fv && ue && vnn) {
             // every flux this column needs is computed here: the loads of a chunk of levels
             // (Hz, u, v only, never the flux arrays being written) are issued together
             // before any of the chunk's arithmetic, the same expressions as below
             // 32-bit element offsets (the launcher takes this form only where (N+1) s2 < 2^31)
             const int s2i = (int)s2, Ii = (int)I;
-            // two chunks per iteration: the second chunk's loads may issue before the first
-            // chunk's arithmetic and stores
-#pragma unroll 2
-            for (int K0 = 0; K0 < N; K0 += (C > 0 ? C : 1)) {
-                constexpr int CC = C > 0 ? C : 1;
+            int o0 = pi, K0 = 0;
+            auto chunk = [&](auto n, auto first) {
+                constexpr int CC = decltype(n)::value;
                 R hz[CC], hzw[CC], hzs[CC], hze[CC], hzn[CC], uu[CC], uE[CC], vv[CC], vN[CC];
 #pragma unroll
                 for (int c = 0; c < CC; ++c) {
-                    const int o = (K0 + c < N ? K0 + c : N - 1) * s2i + pi;
+                    const int o = o0 + c * s2i;
                     hz[c] = Hz[o];
                     hzw[c] = Hz[o - 1];
                     hzs[c] = Hz[o - Ii];
@@ -1464,22 +1464,24 @@ __device__ __forceinline__ void maxflux_omega_body(
                 }
 #pragma unroll
                 for (int c = 0; c < CC; ++c) {
-                    const int K = K0 + c;
-                    if (K < N) {
-                        const int o = K * s2i + pi;
-                        const R hup = (((hz[c] + hzw[c]) * R(0.5)) * uu[c]) * onu;
-                        const R hvp = (((hz[c] + hzs[c]) * R(0.5)) * vv[c]) * omv;
-                        Huon[o] = hup;
-                        Hvom[o] = hvp;
-                        if (K >= 1) {
-                            const R hue = (((hze[c] + hz[c]) * R(0.5)) * uE[c]) * onu_e;
-                            const R hvn = (((hzn[c] + hz[c]) * R(0.5)) * vN[c]) * omv_n;
-                            Wk = Wk - ((hue - hup) + (hvn - hvp));
-                            Wc(K) = Wk;
-                        }
+                    const int o = o0 + c * s2i;
+                    const R hup = (((hz[c] + hzw[c]) * R(0.5)) * uu[c]) * onu;
+                    const R hvp = (((hz[c] + hzs[c]) * R(0.5)) * vv[c]) * omv;
+                    Huon[o] = hup;
+                    Hvom[o] = hvp;
+                    if (!first) {
+                        const R hue = (((hze[c] + hz[c]) * R(0.5)) * uE[c]) * onu_e;
+                        const R hvn = (((hzn[c] + hz[c]) * R(0.5)) * vN[c]) * omv_n;
+                        Wk = Wk - ((hue - hup) + (hvn - hvp));
+                        Wc(K0 + c) = Wk;
                     }
                 }
-            }
+                o0 += CC * s2i;
+                K0 += CC;
+            };
+            // the integral leaves out the lowest level
+            chunk(std::integral_constant<int, 1>(), std::true_type());
+            in_chunks<(C > 0 ? C : 1)>(N - 1, [&](auto n) { chunk(n, std::false_type()); });
         } else {
 #pragma unroll 4
         for (int K = 0; K < N; ++K) {
@@ -1503,24 +1505,19 @@ __device__ __forceinline__ void maxflux_omega_body(
         // 32 for omega alone, 16 after the fluxes (basin4: 0.45 and 0.82 ms; 32 after the
         // fluxes takes 1.14 ms)
         {
-            constexpr int kZ = C < 0 ? 32 : 16;
-            for (int K0 = 1; K0 < N; K0 += kZ) {
+            long o0 = s2 + p;
+            int K0 = 1;
+            in_chunks<(C < 0 ? 32 : 16)>(N - 1, [&](auto n) {
+                constexpr int kZ = decltype(n)::value;
                 R zw[kZ];
 #pragma unroll
-                for (int c = 0; c < kZ; ++c) {
-                    const int K = K0 + c < N ? K0 + c : N - 1;
-                    zw[c] = C > 0 ? z_w[K * (int)s2 + pi] : z_w[(long)K * s2 + p];
-                }
+                for (int c = 0; c < kZ; ++c) zw[c] = z_w[o0 + c * s2];
 #pragma unroll
-                for (int c = 0; c < kZ; ++c) {
-                    const int K = K0 + c;
-                    if (K < N) {
-                        const R wv = Wc(K) - ddiv(Ws * (zw[c] - zbed), h);
-                        if (C > 0) W[K * (int)s2 + pi] = wv;
-                        else W[(long)K * s2 + p] = wv;
-                    }
-                }
-            }
+                for (int c = 0; c < kZ; ++c)
+                    W[o0 + c * s2] = Wc(K0 + c) - ddiv(Ws * (zw[c] - zbed), h);
+                o0 += kZ * s2;
+                K0 += kZ;
+            });
         }
 #undef Wc
         W[(long)N * s2 + p] = R(0);
@@ -2375,19 +2372,23 @@ __global__ void __launch_bounds__(TX *TY) kb_rhs3d(const Member<R> *mt, const in
                                  mb_.y % ntx, mb_.y / ntx);
 }
 
+// Blocks per SM: chunks of 4 levels want 3 (80 registers; with 2 blocks at 128 they take 0.81 ms, with 4 at
+// 64 0.98, on 2050 x 1026 x 50 in FP32, against 0.74), omega alone 4 (FP64 2).
+template <typename R>
+constexpr int mo_blocks(int C) { return C < 0 ? (sizeof(R) == 4 ? 4 : 2) : 3; }
 template <typename R, int C>
-__global__ void __launch_bounds__(kBlock) k_maxflux_omega(
+__global__ void __launch_bounds__(kBlock, mo_blocks<R>(C)) k_maxflux_omega(
     Geo<R> g, const R *__restrict__ u, const R *__restrict__ v, R *Huon, R *Hvom, const R *__restrict__ Hz, R *__restrict__ W, const R *__restrict__ z_w,
     int do_flux, int do_omega, R *__restrict__ zeta1, R *__restrict__ zeta2, const double *__restrict__ Zt) {
     maxflux_omega_body<R, C>(g, u, v, Huon, Hvom, Hz, W, z_w, do_flux, do_omega, zeta1, zeta2, Zt,
                              (long)tid_flat());
 }
-template <typename R>
-__global__ void __launch_bounds__(kBlock) kb_maxflux_omega(
+template <typename R, int C = 0>
+__global__ void __launch_bounds__(kBlock, mo_blocks<R>(C)) kb_maxflux_omega(
     const Member<R> *mt, const int2 *bm, const R *__restrict__ u, const R *__restrict__ v, R *Huon, R *Hvom, const R *__restrict__ Hz,
     R *__restrict__ W, const R *__restrict__ z_w, int do_flux, int do_omega, R *__restrict__ zeta1, R *__restrict__ zeta2, const double *__restrict__ Zt) {
     SF_MEMBER(bm)
-    maxflux_omega_body(g, O3(u), O3(v), O3(Huon), O3(Hvom), ON(Hz), O3(W), O3(z_w), do_flux,
+    maxflux_omega_body<R, C>(g, O3(u), O3(v), O3(Huon), O3(Hvom), ON(Hz), O3(W), O3(z_w), do_flux,
                        do_omega, O2(zeta1), O2(zeta2), O2(Zt), (long)mb_.y * kBlock + threadIdx.x);
 }
 
@@ -2692,13 +2693,16 @@ cudaError_t Ops<R>::maxflux_omega(const sf_ctx *c, const R *u, const R *v, R *Hu
         cudaFuncSetAttribute(k_maxflux_omega<R, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         cudaFuncSetAttribute(k_maxflux_omega<R, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         cudaFuncSetAttribute(k_maxflux_omega<R, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(kb_maxflux_omega<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        for (auto k : {kb_maxflux_omega<R, -1>, kb_maxflux_omega<R, 0>, kb_maxflux_omega<R, 4>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         attr_set[dev] = true;
     }
     if (c->nmem > 1) {
-        kb_maxflux_omega<R><<<c->nbm_pt, kBlock, smem, s>>>(mt<R>(c), c->bm_pt, u, v, Huon, Hvom, Hz,
-                                                           W, z_w, do_flux, do_omega, zeta1, zeta2,
-                                                           Zt);
+        const bool fits = (long)(c->maxN + 1) * c->s2 < (1L << 31);
+        auto k = !do_flux ? kb_maxflux_omega<R, -1>
+                 : fits && c->mo_chunk ? kb_maxflux_omega<R, 4> : kb_maxflux_omega<R, 0>;
+        k<<<c->nbm_pt, kBlock, smem, s>>>(mt<R>(c), c->bm_pt, u, v, Huon, Hvom, Hz, W, z_w, do_flux, do_omega,
+                                         zeta1, zeta2, Zt);
         return cudaGetLastError();
     }
     // the chunked forms address with 32-bit element offsets

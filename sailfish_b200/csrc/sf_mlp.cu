@@ -270,23 +270,32 @@ __global__ void k_colsum(long n, const float *__restrict__ G, float *__restrict_
     atomicAdd(&db[j], s);
 }
 
-// MSE on the first nvalid outputs: dY = 2 (Y - T) / (n * nvalid), loss accumulated into *loss.
-__global__ void k_mse(long n, int nvalid, const float *__restrict__ Y, const float *__restrict__ T,
-                      float *__restrict__ dY, float *loss) {
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// MSE on the first nvalid outputs: dY = 2 (Y - T) / (n * nvalid), loss accumulated into *loss: sums of
+// a thread's elements, then of its block, one atomic per block (at most kMseBlocks of them: each
+// rounds the loss once; an atomic per warp rounded it n * 4 times and serialised in L2).
+// VEC: four elements at a time (buffers on 16-byte boundaries).
+constexpr int kMseBlocks = 592;
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_mse(long n, int nvalid, const float *__restrict__ Y,
+                                             const float *__restrict__ T, float *__restrict__ dY, float *loss) {
+    constexpr int E = VEC ? 4 : 1;
+    using V = std::conditional_t<VEC, float4, float>;
     float l = 0.f;
-    if (e < n * kTile) {
-        const int j = (int)(e % kTile);
-        float g = 0.f;
-        if (j < nvalid) {
-            const float d = Y[e] - T[e];
-            g = 2.f * d / (float)(n * nvalid);
-            l = d * d / (float)(n * nvalid);
+    const float scale = (float)(n * nvalid);
+#pragma unroll 2
+    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n * (kTile / E); e += (long)gridDim.x * blockDim.x) {
+        const V y = reinterpret_cast<const V *>(Y)[e], t = reinterpret_cast<const V *>(T)[e];
+        V g;
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const bool in = (int)(e % (kTile / E)) * E + q < nvalid;
+            const float d = in ? reinterpret_cast<const float *>(&y)[q] - reinterpret_cast<const float *>(&t)[q] : 0.f;
+            reinterpret_cast<float *>(&g)[q] = 2.f * d / scale;
+            l += d * d / scale;
         }
-        dY[e] = g;
+        reinterpret_cast<V *>(dY)[e] = g;
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    // one atomic per block: an atomic per warp on the one loss word serialised in L2
     __shared__ float part[8];
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = l;
     __syncthreads();
@@ -1453,7 +1462,10 @@ int sf_mlp_backward(const sf_mlp_params *w, int n, const float *X, const float *
 
 int sf_mlp_mse(int n, int nvalid, const float *Y, const float *T, float *dY, float *loss, sf_stream s) {
     if (n <= 0 || !Y || !T || !dY || !loss) return mfail(SF_EINVAL, "bad argument");
-    sf::mlp::k_mse<<<nblk((long)n * kTile, 256), 256, 0, S(s)>>>(n, nvalid, Y, T, dY, loss);
+    const bool vec = aligned16(Y) && aligned16(T) && aligned16(dY);
+    const unsigned nb = nblk((long)n * kTile / (vec ? 4 : 1), 256);
+    (vec ? sf::mlp::k_mse<true> : sf::mlp::k_mse<false>)<<<nb < sf::mlp::kMseBlocks ? nb : sf::mlp::kMseBlocks, 256, 0,
+                                                           S(s)>>>(n, nvalid, Y, T, dY, loss);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_mse");
 }

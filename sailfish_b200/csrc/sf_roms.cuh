@@ -503,49 +503,80 @@ __device__ __forceinline__ void roms_acc_at(const Geo<R> &g, const RomsArgs<R> &
 // fluxes UFx = (Huon_i + Huon_i+1)/4 (u_i + u_i+1) at rho points and UFe = (Hvom_i +
 // Hvom_i-1)/4 (u_j + u_j-1) at psi points (the UV_C2ADVECTION form of the reference's ROMS
 // transcription, obsolete/step2d_LF_AM3.h.py:1244-1300, per level), V alike; the vertical
-// advection is implicit, in the column solve (roms_column).  One thread per rho point p (its
-// west U face and south V face), levels in order; the expressions keep the oracle's operand
-// order (oracle/roms_oracle.py, rhs3d).
+// advection is implicit, in the column solve (roms_column).  The expressions keep the oracle's
+// operand order (oracle/roms_oracle.py, rhs3d).
+//
+// A warp takes a strip of 29 columns (lanes 1 .. 29; 0 and 30 their neighbours) of one level and
+// walks up its rows: every field is loaded once per node, west and east by shuffle, the southern
+// fluxes from the row before, the next row's loads in flight.  Bound: the 28 bytes a point and level
+// in FP32 (0.45 ms for 2050 x 1026 x 50 at the copy bandwidth); a thread per column loading some 25
+// neighbour values a level took 1.19 ms.
 template <typename R>
-__device__ __forceinline__ void roms_rhs3d_at(const Geo<R> &g, const R *__restrict__ u,
-                                              const R *__restrict__ v, const R *__restrict__ Hu,
-                                              const R *__restrict__ Hv, const R *__restrict__ Hz,
-                                              R *__restrict__ ru, R *__restrict__ rv,
-                                              const long p) {
-    if (p >= g.s2) return;
-    const int j = fdiv((int)p, g.dI), i = (int)p - j * g.I;
-    const long I = g.I, s2 = g.s2;
-    const int N = g.N;
-    const bool uf = i >= 2 && i <= g.I - 2 && j >= 1 && j <= g.J - 2;
-    const bool vf = j >= 2 && j <= g.J - 2 && i >= 1 && i <= g.I - 2;
-    const R *fomn = g.fomn;
-    for (int k = 0; k <= N; ++k) {
-        const long o = (long)k * s2;
-        R tu = R(0), tv = R(0);
-        if (k < N && uf) {
-            const R *uk = u + o, *vk = v + o, *hu = Hu + o, *hv = Hv + o, *hz = Hz + o;
-            const R UFp = (hz[p] * fomn[p]) * ((vk[p] + vk[p + I]) * R(0.5));
-            const R UFw = (hz[p - 1] * fomn[p - 1]) * ((vk[p - 1] + vk[p - 1 + I]) * R(0.5));
-            const R cor = (UFp + UFw) * R(0.5);
-            const R Xp = (R(0.25) * (hu[p] + hu[p + 1])) * (uk[p] + uk[p + 1]);
-            const R Xw = (R(0.25) * (hu[p - 1] + hu[p])) * (uk[p - 1] + uk[p]);
-            const R En = (R(0.25) * (hv[p + I] + hv[p + I - 1])) * (uk[p + I] + uk[p]);
-            const R Es = (R(0.25) * (hv[p] + hv[p - 1])) * (uk[p] + uk[p - I]);
-            tu = cor - ((Xp - Xw) + (En - Es));
+struct RhsRow {
+    R u, v, hu, hv, hz, fo;
+};
+template <typename R>
+__device__ __forceinline__ void roms_rhs3d_rows(const Geo<R> &g, const R *__restrict__ u,
+                                                const R *__restrict__ v, const R *__restrict__ Hu,
+                                                const R *__restrict__ Hv, const R *__restrict__ Hz,
+                                                R *__restrict__ ru, R *__restrict__ rv, const int i0,
+                                                const int j0, const int nrows, const int k) {
+    const int I = g.I, J = g.J, lane = threadIdx.x & 31;
+    if (j0 >= J) return;   // whole warp
+    const int i = i0 - 1 + lane, il = i < 0 ? 0 : (i > I - 1 ? I - 1 : i);
+    const bool out = lane >= 1 && lane <= kRomsCols && i < I;
+    const int jend = j0 + nrows < J ? j0 + nrows : J;
+    const long o = (long)k * g.s2;
+    if (k >= g.N) {   // the level above the surface
+        if (out)
+            for (int j = j0; j < jend; ++j) {
+                ru[o + j * I + i] = R(0);
+                rv[o + j * I + i] = R(0);
+            }
+        return;
+    }
+    u += o;
+    v += o;
+    Hu += o;
+    Hv += o;
+    Hz += o;
+    ru += o;
+    rv += o;
+    auto west = [](R x) { return __shfl_up_sync(0xffffffffu, x, 1); };
+    auto east = [](R x) { return __shfl_down_sync(0xffffffffu, x, 1); };
+    auto load = [&](int j) {
+        const int p = (j < 0 ? 0 : (j > J - 1 ? J - 1 : j)) * I + il;
+        return RhsRow<R>{u[p], v[p], Hu[p], Hv[p], Hz[p], g.fomn[p]};
+    };
+    RhsRow<R> c = load(j0 - 1), n = load(j0);
+    R hus = R(0), es = R(0), vfs = R(0), eps = R(0);   // the row below: Hu, its northern fluxes
+    for (int j = j0 - 1; j < jend; ++j) {
+        const RhsRow<R> nn = load(j + 2);   // in flight
+        const R ue = east(c.u), vw = west(c.v);
+        // factors of the Coriolis terms and of the momentum fluxes; differences and sums of two products
+        // with the contraction written out (rfma)
+        const R cf = rmul(c.hz, c.fo), vb = rmul(c.v + n.v, R(0.5)), ub = rmul(c.u + ue, R(0.5));
+        const R vf = rmul(cf, ub);
+        const R hu = rmul(R(0.25), c.hu + east(c.hu)), wu = c.u + ue;           // at rho points
+        const R hn = rmul(R(0.25), n.hv + west(n.hv)), yn = n.u + c.u, en = rmul(hn, yn);   // at psi points
+        const R hx = rmul(R(0.25), c.hu + hus), wx = c.v + vw, xv = rmul(hx, wx);
+        const R hp = rmul(R(0.25), c.hv + n.hv), yp = c.v + n.v, ep = rmul(hp, yp);
+        const R ufw = west(rmul(cf, vb)), xuw = west(rmul(hu, wu)), hxe = east(hx), wxe = east(wx);
+        if (j >= j0 && out) {
+            R tu = R(0), tv = R(0);
+            if (i >= 2 && i <= I - 2 && j >= 1 && j <= J - 2)
+                tu = rmul(rfma(cf, vb, ufw), R(0.5)) - (rfma(hu, wu, -xuw) + rfma(hn, yn, -es));
+            if (j >= 2 && j <= J - 2 && i >= 1 && i <= I - 2)
+                tv = -rmul(rfma(cf, ub, vfs), R(0.5)) - (rfma(hxe, wxe, -xv) + rfma(hp, yp, -eps));
+            ru[j * I + i] = tu;
+            rv[j * I + i] = tv;
         }
-        if (k < N && vf) {
-            const R *uk = u + o, *vk = v + o, *hu = Hu + o, *hv = Hv + o, *hz = Hz + o;
-            const R VFp = (hz[p] * fomn[p]) * ((uk[p] + uk[p + 1]) * R(0.5));
-            const R VFs = (hz[p - I] * fomn[p - I]) * ((uk[p - I] + uk[p - I + 1]) * R(0.5));
-            const R cor = -((VFp + VFs) * R(0.5));
-            const R Xe = (R(0.25) * (hu[p + 1] + hu[p + 1 - I])) * (vk[p + 1] + vk[p]);
-            const R Xw = (R(0.25) * (hu[p] + hu[p - I])) * (vk[p] + vk[p - 1]);
-            const R Ep = (R(0.25) * (hv[p] + hv[p + I])) * (vk[p] + vk[p + I]);
-            const R Es = (R(0.25) * (hv[p - I] + hv[p])) * (vk[p - I] + vk[p]);
-            tv = cor - ((Xe - Xw) + (Ep - Es));
-        }
-        ru[o + p] = tu;
-        rv[o + p] = tv;
+        es = en;
+        vfs = vf;
+        eps = ep;
+        hus = c.hu;
+        c = n;
+        n = nn;
     }
 }
 
@@ -886,17 +917,23 @@ __global__ void __launch_bounds__(256) kb_roms_acc(const Member<R> *mt, const in
     roms_acc_at(m.g, roms_args_at(a, m.o2), m.p);
 }
 template <typename R>
-__global__ void __launch_bounds__(256) k_roms_rhs3d(Geo<R> g, const R *u, const R *v, const R *Hu,
-                                                    const R *Hv, const R *Hz, R *ru, R *rv) {
-    roms_rhs3d_at(g, u, v, Hu, Hv, Hz, ru, rv, tid_flat());
+__global__ void __launch_bounds__(32 * kRomsWarps) k_roms_rhs3d(Geo<R> g, const R *u, const R *v, const R *Hu,
+                                                                const R *Hv, const R *Hz, R *ru, R *rv,
+                                                                int nrows) {
+    roms_rhs3d_rows(g, u, v, Hu, Hv, Hz, ru, rv, (int)blockIdx.x * kRomsCols,
+                    ((int)blockIdx.y * kRomsWarps + (int)(threadIdx.x >> 5)) * nrows, nrows, (int)blockIdx.z);
 }
 template <typename R>
-__global__ void __launch_bounds__(256) kb_roms_rhs3d(const Member<R> *mt, const int2 *bm,
-                                                     const R *u, const R *v, const R *Hu,
-                                                     const R *Hv, const R *Hz, R *ru, R *rv) {
-    const MemberAt<R> m = member_at(mt, bm, 256);
-    roms_rhs3d_at(m.g, u + m.o3, v + m.o3, Hu + m.o3, Hv + m.o3, Hz + m.oN, ru + m.o3, rv + m.o3,
-                  m.p);
+__global__ void __launch_bounds__(32 * kRomsWarps) kb_roms_rhs3d(const Member<R> *mt, const int2 *bm, const R *u,
+                                                                 const R *v, const R *Hu, const R *Hv,
+                                                                 const R *Hz, R *ru, R *rv, int nrows) {
+    const int2 mb = bm[blockIdx.x];
+    const Member<R> &M = mt[mb.x];
+    if ((int)blockIdx.y > M.g.N) return;
+    const int ns = (M.g.I + kRomsCols - 1) / kRomsCols, by = mb.y / ns, bx = mb.y - by * ns;
+    const long o3 = M.off3;
+    roms_rhs3d_rows(M.g, u + o3, v + o3, Hu + o3, Hv + o3, Hz + M.offN, ru + o3, rv + o3, bx * kRomsCols,
+                    (by * kRomsWarps + (int)(threadIdx.x >> 5)) * nrows, nrows, (int)blockIdx.y);
 }
 template <typename R>
 __global__ void __launch_bounds__(256) k_roms_stress3d(Geo<R> g, const R *u, const R *v, R *ru,
@@ -993,10 +1030,18 @@ cudaError_t Ops<R>::roms_stress3d(const sf_ctx *c, const R *u, const R *v, R *ru
 template <typename R>
 cudaError_t Ops<R>::roms_rhs3d(const sf_ctx *c, const R *u, const R *v, const R *Huon,
                                const R *Hvom, const R *Hz, R *ru, R *rv, cudaStream_t s) {
-    if (c->nmem > 1)
-        kb_roms_rhs3d<R><<<c->nbm_pt, 256, 0, s>>>(mt<R>(c), c->bm_pt, u, v, Huon, Hvom, Hz, ru, rv);
-    else
-        k_roms_rhs3d<R><<<blocks_for(c->s2, 256), 256, 0, s>>>(geo(c), u, v, Huon, Hvom, Hz, ru, rv);
+    const int B = 32 * kRomsWarps;
+    if (c->nmem > 1) {
+        kb_roms_rhs3d<R><<<dim3(c->nbm_roms, c->maxN + 1), B, 0, s>>>(mt<R>(c), c->bm_roms, u, v, Huon, Hvom, Hz, ru,
+                                                                     rv, c->roms_rows);
+    } else {
+        // rows a warp walks: 8 (1026 x 514 x 50 in FP32: 4, 8, 16, 32, 64 rows 0.177, 0.158, 0.162, 0.168,
+        // 0.184 ms), 32 on large grids (2050 x 1026 x 50: 0.685, 0.618, 0.627, 0.605, 0.584)
+        const int rows = c->s2 >= (1L << 20) ? 32 : 8;
+        const dim3 grid((c->I + kRomsCols - 1) / kRomsCols, (c->J + rows * kRomsWarps - 1) / (rows * kRomsWarps),
+                        c->N + 1);
+        k_roms_rhs3d<R><<<grid, B, 0, s>>>(geo(c), u, v, Huon, Hvom, Hz, ru, rv, rows);
+    }
     return cudaGetLastError();
 }
 template <typename R>
