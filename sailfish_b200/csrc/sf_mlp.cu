@@ -377,6 +377,22 @@ __device__ __forceinline__ void store_act8x4(__nv_bfloat16 *sA, int r, int n0, c
     }
 }
 
+// A layer's 128 x 128 weights into the core-matrix layout: 16 bytes a load (a warp takes 8 rows x 64
+// bytes, so its shared stores fill whole core matrices), element by element off 16-byte boundaries.
+template <int THREADS>
+__device__ __forceinline__ void stage_layer(__nv_bfloat16 *dst, const __nv_bfloat16 *__restrict__ W) {
+    if ((reinterpret_cast<uintptr_t>(W) & 15) == 0) {
+#pragma unroll
+        for (int q = 0; q < kTile * kTile / 8 / THREADS; ++q) {
+            const int e = threadIdx.x + q * THREADS, l = e & 31, w = e >> 5;
+            const int r = (w >> 2) * 8 + (l & 7), k = ((w & 3) * 4 + (l >> 3)) * 8;
+            *reinterpret_cast<uint4 *>(&dst[cm_index(r, k)]) = *reinterpret_cast<const uint4 *>(W + r * kTile + k);
+        }
+    } else {
+        for (int e = threadIdx.x; e < kTile * kTile; e += THREADS) dst[cm_index(e >> 7, e & 127)] = W[e];
+    }
+}
+
 template <int ACT>
 __global__ void __launch_bounds__(kInferThreads, 1) k_infer(InferW w, long n,
                                                             const float *__restrict__ X,
@@ -394,8 +410,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_infer(InferW w, long n,
         asm volatile("fence.mbarrier_init.release.cluster;" ::);
     }
     for (int l = 0; l < SF_MLP_LAYERS; ++l) {
-        for (int e = tid; e < kTile * kTile; e += kInferThreads)
-            sW[l * kTile * kTile + cm_index(e >> 7, e & 127)] = w.W[l][e];
+        stage_layer<kInferThreads>(sW + l * kTile * kTile, w.W[l]);
         for (int e = tid; e < kTile; e += kInferThreads) sbias[l][e] = w.b[l] ? w.b[l][e] : 0.f;
     }
     fence_before();
@@ -1173,8 +1188,7 @@ __global__ void __launch_bounds__(kClosureThreads, 1) k_closure_mlp(Geo<R> g, In
                           &xbar[b]);
     }
     for (int l = 0; l < SF_MLP_LAYERS; ++l) {
-        for (int e = tid; e < kTile * kTile; e += kClosureThreads)
-            sW[l * kTile * kTile + cm_index(e >> 7, e & 127)] = w.W[l][e];
+        stage_layer<kClosureThreads>(sW + l * kTile * kTile, w.W[l]);
         for (int e = tid; e < kTile; e += kClosureThreads) sbias[l][e] = w.b[l] ? w.b[l][e] : 0.f;
     }
     fence_before();
