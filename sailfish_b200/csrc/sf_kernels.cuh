@@ -2068,18 +2068,19 @@ __device__ __forceinline__ void step3d_uv_pipe_body(const Geo<R> &g, float *__re
         const float sub = (float)((O - dbar) / H);
         float x = ddp;
         outc[(N - 1) * s2i] = x - sub;
-        for (int k = N - 2; k >= 0; k -= kBackChunk) {
-            float dv[kBackChunk];   // the chunk's d' first (independent loads), then the chain
+        int k = N - 2;
+        in_chunks<kBackChunk>(N - 1, [&](auto n) {
+            constexpr int C = decltype(n)::value;
+            float dv[C];   // the chunk's d' first (independent loads), then the chain
 #pragma unroll
-            for (int h = 0; h < kBackChunk; ++h) dv[h] = k - h >= 0 ? outc[(k - h) * s2i] : 0.f;
+            for (int h = 0; h < C; ++h) dv[h] = outc[(k - h) * s2i];
 #pragma unroll
-            for (int h = 0; h < kBackChunk; ++h) {
-                if (k - h >= 0) {
-                    x = dv[h] - cc[(k - h) * kPipeThreads] * x;
-                    outc[(k - h) * s2i] = x - sub;
-                }
+            for (int h = 0; h < C; ++h) {
+                x = dv[h] - cc[(k - h) * kPipeThreads] * x;
+                outc[(k - h) * s2i] = x - sub;
             }
-        }
+            k -= C;
+        });
         // sum_k hz_k (x_k - sub) from the column identity
         const double Hx = Rs + (double)fc0 * (double)x - (double)sub * H;
         const float bar = (float)(dbar / H + (Hx - dbar) / H);
