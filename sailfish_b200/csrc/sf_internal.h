@@ -191,13 +191,15 @@ struct sf_ctx {
 
 namespace sf {
 
-// Kernels launched through launch_dep (programmatic dependent launch) start with pdl_enter():
-// it lets the next kernel on the stream begin launching its blocks, then waits until this
-// kernel's predecessor has completed and its writes are visible.  Both are no-ops when the
-// kernel was launched without the attribute.
+// Kernels launched through launch_dep (programmatic dependent launch) start with pdl_enter(): they
+// wait until their predecessor has completed and its writes are visible, and let the next kernel on
+// the stream begin launching its blocks only then, so that at most one launch waits in the SMs and the
+// running one's blocks spread over all of them (the other way round blocks of several waiting
+// launches take the places: the reference form's loop on 514 x 258 in FP32 1.45 ms against 1.38).
+// Both are no-ops when the kernel was launched without the attribute.
 __device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <typename... KArgs, typename... Args>

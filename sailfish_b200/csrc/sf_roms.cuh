@@ -23,17 +23,6 @@
 namespace sf {
 
 
-// The barotropic phases are launched with programmatic dependent launch (as the reference form's
-// loop): a kernel's blocks become resident while its predecessor runs and wait for its completion on
-// the device.  They let their own successor in only after that wait: at most one launch waits in
-// the SMs, so that the running one's blocks spread over all of them (with the order the other way
-// round blocks of several waiting launches take the places: 258 x 130 nodes in FP32, 6.9 us a substep
-// against 3.4).
-__device__ __forceinline__ void pdl_wait_then_launch() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // The barotropic substep's products and sums, with the FP32 form's contractions written out: a product
 // either rounds by itself (rmul) or goes into one fused multiply-add (rfma), so that every form of
 // the substep (two launches, fused; single grid, ensemble) gives the same bits whatever the compiler
@@ -327,7 +316,7 @@ __device__ __forceinline__ void roms_sub_tile(const Geo<R> &g, const RomsArgs<R>
     // the context's metrics do not depend on the kernels before: loaded while those finish
     const R h = g.h[q], hs = g.h[qs], hn = g.h[qn], om = g.om_v[q], omN = g.om_v[qn];
     const R on = g.on_u[q], pm = g.pm[q], pn = g.pn[q], fo = g.fomn[q];
-    pdl_wait_then_launch();
+    pdl_enter();
     // LATE: values needed late wait in shared memory (averages; the old level's velocities, stresses,
     // tendencies), which leaves registers for more blocks per SM; else in registers
     constexpr int T = 32 * H;
@@ -849,14 +838,14 @@ __device__ __forceinline__ RomsArgs<R> roms_args_at(const RomsArgs<R> &a, long o
 
 template <typename R, int PH>
 __global__ void __launch_bounds__(32 * kRomsWarps) k_roms_phase(Geo<R> g, RomsArgs<R> a, int nrows) {
-    pdl_wait_then_launch();
+    pdl_enter();
     roms_phase_rows<R, PH>(g, a, (int)blockIdx.x * kRomsCols,
                            ((int)blockIdx.y * kRomsWarps + (int)(threadIdx.x >> 5)) * nrows, nrows);
 }
 template <typename R, int PH>
 __global__ void __launch_bounds__(32 * kRomsWarps) kb_roms_phase(const Member<R> *mt, const int2 *bm,
                                                                  RomsArgs<R> a, int nrows) {
-    pdl_wait_then_launch();
+    pdl_enter();
     const int2 mb = bm[blockIdx.x];
     const Member<R> &M = mt[mb.x];
     const int ns = (M.g.I + kRomsCols - 1) / kRomsCols, by = mb.y / ns, bx = mb.y - by * ns;
@@ -907,12 +896,12 @@ cudaError_t roms_sub_launch(const sf_ctx *c, const RomsArgs<R> &a, dim3 grid, cu
 }
 template <typename R>
 __global__ void __launch_bounds__(256) k_roms_acc(Geo<R> g, RomsArgs<R> a) {
-    pdl_wait_then_launch();
+    pdl_enter();
     roms_acc_at(g, a, tid_flat());
 }
 template <typename R>
 __global__ void __launch_bounds__(256) kb_roms_acc(const Member<R> *mt, const int2 *bm, RomsArgs<R> a) {
-    pdl_wait_then_launch();
+    pdl_enter();
     const MemberAt<R> m = member_at(mt, bm, 256);
     roms_acc_at(m.g, roms_args_at(a, m.o2), m.p);
 }
