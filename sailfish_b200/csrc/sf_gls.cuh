@@ -64,6 +64,20 @@ __device__ __forceinline__ R gls_pow(R x, GlsExp e) {
     return e.h < 0 ? R(1) / r : r;
 }
 
+// gls_pow with 2 e known to the compiler (H), or read from e (kGlsPow).
+template <int H, typename R>
+__device__ __forceinline__ R gls_powc(R x, GlsExp e) {
+    if constexpr (H == kGlsPow) {
+        return gls_pow(x, e);
+    } else {
+        constexpr int a = H < 0 ? -H : H, n = a >> 1;
+        static_assert(n <= 3, "x, x^2, x^3 and their halves");
+        R r = n == 0 ? R(1) : n == 1 ? x : n == 2 ? x * x : x * (x * x);
+        if constexpr (a & 1) r = n ? sqrt(x) * r : sqrt(x);
+        return H < 0 ? R(1) / r : r;
+    }
+}
+
 // The model's constants, evaluated once on the host in FP64 (a column evaluated a dozen powers of
 // them), and its exponents.
 template <typename R>
@@ -125,16 +139,21 @@ GlsConst<R> gls_const(const sf_gls_params &P, double dt) {
 // sets (a limit on psi in the reference's text) is compared as a length, without one.
 // Blocks per SM: the levels are a chain of divisions and roots, so warps hide the latency, not loads in
 // flight (levels in chunks of 4 at 128 registers: 0.97 and 0.41 ms for the two cases above; one at a
-// time with 10 blocks at 48 registers in FP32, 7 at 72 in FP64: 0.76 and 0.31; 12 blocks 0.88).
+// time with 10 blocks at 48 registers in FP32, 7 at 72 in FP64: 0.76 and 0.31, 0.68 and 0.30 now; 12 blocks 0.88).
 template <typename R>
 constexpr int gls_blocks() { return sizeof(R) == 4 ? 10 : 7; }
-template <typename R, typename Off>
+// KEPS: the exponents of k-epsilon, the default model (m = 3/2, n = -1), as constants: the branches on
+// each exponent and its cases leave the level loops. 1024x512x50 FP32 0.760 ms -> 0.683, 512x256x32 FP64
+// 0.231 -> 0.202; a model with other exponents takes the other variant (gen: 0.800 and 0.303).
+template <typename R, typename Off, bool KEPS>
 __global__ void __launch_bounds__(128, gls_blocks<R>()) k_gls_corrector(
     Geo<R> g, const GlsConst<R> G, const R *__restrict__ u, const R *__restrict__ v, const R *__restrict__ z_r,
     const R *__restrict__ Hz, const R *__restrict__ bvf, const R *__restrict__ sustr,
     const R *__restrict__ svstr, R *tke, R *gls, R *Akv, R *Akt, R *Akk, R *Akp, R *Lscale,
     const R *__restrict__ tkn0, const R *__restrict__ gln0, const uint8_t *__restrict__ sel,
     const int *__restrict__ list, const int *__restrict__ count) {
+    constexpr int kM = KEPS ? 3 : kGlsPow, kN = KEPS ? -2 : kGlsPow, kI = KEPS ? -2 : kGlsPow,
+                  kMi = KEPS ? 2 : kGlsPow, kN1 = KEPS ? -4 : kGlsPow;
     int pi = (int)tid_flat();
     if (list) {                    // a compacted list of columns: thread t takes list[t]
         if (pi >= *count) return;
@@ -186,7 +205,7 @@ __global__ void __launch_bounds__(128, gls_blocks<R>()) k_gls_corrector(
         // Hz_w * tke/gls(nstp) (the predictor's start without the advective terms)
         const R tr = (tkn0 ? tkn0[o] : cffz * tko) + dt * cffz * Kprod;
         const R gr = (gln0 ? gln0[o] : cffz * glo) + dt * cffz * Pprod * glo / fmax(tko, Kmin);
-        const R diss = G.cmu_fac2 * gls_pow(glo / gls_pow(tko, G.m), G.mi) * sqrt(tko);
+        const R diss = G.cmu_fac2 * gls_powc<kMi>(glo / gls_powc<kM>(tko, G.m), G.mi) * sqrt(tko);
         const R bck = cffz * (R(1) + dt * diss + dt * sk / tko) - fk - fk1;
         const R bcp = cffz * (R(1) + dt * G.c2 * diss + dt * sp / tko) - fp - fp1;
         // tke (:571-604) and gls (:608-656) eliminated
@@ -228,8 +247,8 @@ __global__ void __launch_bounds__(128, gls_blocks<R>()) k_gls_corrector(
     const R bu = bustr(p) + bustr(p + 1), bv = bvstr(p) + bvstr(p + I);
     const R tkN = fmax(G.cmu_fac3 * R(0.5) * sqrt(su * su + sv * sv), Kmin);
     const R tk0 = fmax(G.cmu_fac3 * R(0.5) * sqrt(bu * bu + bv * bv), Kmin);
-    const R glN = fmax(gls_pow(tkN, G.m) * G.glsN, Pmin);
-    const R gl0 = fmax(G.gls0 * gls_pow(tk0, G.m), Pmin);
+    const R glN = fmax(gls_powc<kM>(tkN, G.m) * G.glsN, Pmin);
+    const R gl0 = fmax(G.gls0 * gls_powc<kM>(tk0, G.m), Pmin);
     // --- up: tke
     o = p + s2;
     tk = fmax(tk, Kmin);
@@ -254,9 +273,9 @@ __global__ void __launch_bounds__(128, gls_blocks<R>()) k_gls_corrector(
     };
     in_chunks<4>(N - 2, up);
     // fluxes of gls through the surface and the bottom (:608-630)
-    const R fluxt = G.fluxt * gls_pow(R(0.5) * (tkN + tk), G.m) *
-                    gls_pow(G.Zos + R(0.5) * Hz[p + (Off)(N - 1) * s2], G.n1) * akpN;
-    const R fluxb = G.fluxb * gls_pow(R(0.5) * (tk0 + tk1), G.m) * gls_pow(R(0.5) * Hz[p] + G.Zob, G.n1) * AkpB;
+    const R fluxt = G.fluxt * gls_powc<kM>(R(0.5) * (tkN + tk), G.m) *
+                    gls_powc<kN1>(G.Zos + R(0.5) * Hz[p + (Off)(N - 1) * s2], G.n1) * akpN;
+    const R fluxb = G.fluxb * gls_powc<kM>(R(0.5) * (tk0 + tk1), G.m) * gls_powc<kN1>(R(0.5) * Hz[p] + G.Zob, G.n1) * AkpB;
     // --- up: gls and the mixing coefficients (:662-825); the old values of a level are read before they
     // are written
     const R sqrt2 = sqrt(R(2));
@@ -266,8 +285,8 @@ __global__ void __launch_bounds__(128, gls_blocks<R>()) k_gls_corrector(
         const R a = gls[o], b = Akp[o], f = Akk[o], t = Akt[o], b2 = bvf[o], ls = Lscale[o], to = tke[o];
         gl = (a - fluxt * b) - (k == 1 ? gl : f * gl);
         const R b2p = fmax(R(0), b2);
-        const R tkn = fmax(t, Kmin), tm = gls_pow(tkn, G.m);
-        const R Ls_gl = G.cmu_fac1 * gls_pow(fmax(gl, Pmin) / tm, G.in);
+        const R tkn = fmax(t, Kmin), tm = gls_powc<kM>(tkn, G.m);
+        const R Ls_gl = G.cmu_fac1 * gls_powc<kI>(fmax(gl, Pmin) / tm, G.in);
         const R Ls_unlmt = fmax(eps, fmin(Ls_gl, sqrt(R(0.56) * tkn) / (sqrt(b2p) + eps)));
         const R Ls = b2 > R(0) ? fmin(Ls_unlmt, sqrt(R(0.56) * tkn / (b2p + eps))) : Ls_unlmt;
         R Gh = fmin((R)kGh0, -b2 * Ls * Ls / (R(2) * tkn));
@@ -282,7 +301,7 @@ __global__ void __launch_bounds__(128, gls_blocks<R>()) k_gls_corrector(
         Akp[o] = G.Akp_bak + Sm * ql * G.ogls_sigp;
         Lscale[o] = Ls;
         tke[o] = tkn;
-        gls[o] = fmax(G.cmu0p * tm * gls_pow(Ls, G.n), Pmin);
+        gls[o] = fmax(G.cmu0p * tm * gls_powc<kN>(Ls, G.n), Pmin);
         o += s2;
     }
     const R AvN = G.Akv_bak + (R)kVonKar * G.Zos * G.cmu0 * sqrt(tkN);

@@ -2812,7 +2812,10 @@ cudaError_t Ops<R>::gls_corrector(const sf_ctx *c, const sf_gls_params &P, doubl
                                   const R *gln0, const uint8_t *sel, const int *list,
                                   const int *count, cudaStream_t s) {
     const bool fits = (long)(c->N + 2) * c->s2 < (1L << 31);   // 32-bit element offsets
-    (fits ? k_gls_corrector<R, int> : k_gls_corrector<R, long>)<<<blocks_for(c->s2, 128), 128, 0, s>>>(
+    const bool ke = P.m == 1.5 && P.n == -1.0;                  // exponents as constants: see KEPS
+    auto k = fits ? (ke ? k_gls_corrector<R, int, true> : k_gls_corrector<R, int, false>)
+                  : (ke ? k_gls_corrector<R, long, true> : k_gls_corrector<R, long, false>);
+    k<<<blocks_for(c->s2, 128), 128, 0, s>>>(
         geo(c), gls_const<R>(P, dt), u, v, z_r, Hz, bvf, sustr, svstr, tke, gls, Akv, Akt, Akk, Akp, Lscale,
         tkn0, gln0, sel, list, count);
     return cudaGetLastError();

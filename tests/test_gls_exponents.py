@@ -22,3 +22,14 @@ def test_exponents_match_oracle(p, m, n, N):
     got = gpu_run(c, "fp64", preset=P)
     for k in FIELDS:
         np.testing.assert_allclose(got[k], ref[k], rtol=1e-9, atol=0, err_msg=k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [5, 8, 9, 64])
+def test_k_epsilon_constants_match_oracle(N):
+    """The default model's own variant: remainders of the level chunks, the shortest and longest column."""
+    c = make(N=N, seed=20 + N)
+    ref = dict(zip(FIELDS, run_oracle(c)))
+    got = gpu_run(c, "fp64")
+    for k in FIELDS:
+        np.testing.assert_allclose(got[k], ref[k], rtol=1e-9, atol=0, err_msg=k)
