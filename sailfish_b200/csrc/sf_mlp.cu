@@ -1009,6 +1009,9 @@ __global__ void k_apply(Geo<R> g, const float *__restrict__ Y, const uint8_t *__
 // issued for the next tile as soon as the last layer's products have read the current one, so
 // it overlaps the output epilogue; the epilogue writes Akv/Akt level by level (lanes along the
 // columns: coalesced) for the interior columns in range.
+// k_closure_mlp is a dependent launch: its CTAs take SMs as the last feature-row blocks leave them and
+// load the weights (160 KB) before they wait for the rows (FP32, N = 50: 1024 x 512 columns 337 -> 330 us,
+// 256 x 128 51 -> 48.6, 128 x 64 46 -> 36; 334, 48.7 and 43.5 without the early trigger).
 template <typename R>
 __global__ void __launch_bounds__(128) k_closure_rows(Geo<R> g, const R *__restrict__ u,
         const R *__restrict__ v, const R *__restrict__ z_r, const R *__restrict__ bvf,
@@ -1016,6 +1019,8 @@ __global__ void __launch_bounds__(128) k_closure_rows(Geo<R> g, const R *__restr
         const float *__restrict__ lo, const float *__restrict__ hi, uint8_t *__restrict__ fallback,
         int *__restrict__ flist, int *__restrict__ fcount, __nv_bfloat16 *__restrict__ Xt, long nrows) {
     __shared__ float slo[kTile], shi[kTile];   // the range box, read by every feature check
+    // k_closure_mlp may take the SMs that the last blocks leave (it waits for this grid before Xt)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (int f = threadIdx.x; f < kTile; f += blockDim.x) {
         slo[f] = f < nfeat ? lo[f] : 0.f;
         shi[f] = f < nfeat ? hi[f] : 0.f;
@@ -1182,14 +1187,19 @@ __global__ void __launch_bounds__(kClosureThreads, 1) k_closure_mlp(Geo<R> g, In
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::);
         fence_proxy_async();
-        for (int b = 0; b < 2; ++b)   // each group's first operand, while the weights load
-            if (tile_of(b) < ntiles)
-                bulk_load(sA0 + b * kTile * kTile, Xt + tile_of(b) * kTile * kTile, kTile * kTile * 2,
-                          &xbar[b]);
     }
+    // The weights: written before k_closure_rows began, which waited for all before it.
     for (int l = 0; l < SF_MLP_LAYERS; ++l) {
         stage_layer<kClosureThreads>(sW + l * kTile * kTile, w.W[l]);
         for (int e = tid; e < kTile; e += kClosureThreads) sbias[l][e] = w.b[l] ? w.b[l][e] : 0.f;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // Xt and fallback
+    if (tid == 0) {
+        fence_proxy_async();
+        for (int b = 0; b < 2; ++b)   // each group's first operand
+            if (tile_of(b) < ntiles)
+                bulk_load(sA0 + b * kTile * kTile, Xt + tile_of(b) * kTile * kTile, kTile * kTile * 2,
+                          &xbar[b]);
     }
     fence_before();
     __syncthreads();
@@ -1629,20 +1639,21 @@ int sf_closure_step(sf_ctx *c, const sf_mlp_params *w, const void *u, const void
             g, (const double *)u, (const double *)v, (const double *)z_r, (const double *)bvf,
             (const double *)sustr, (const double *)svstr, nfeat, lo, hi, fallback, fallback_list,
             fallback_count, X, nrows);
-        (relu ? k_closure_mlp<double, kActRelu> : k_closure_mlp<double, kActGelu>)
-            <<<grid, sf::mlp::kClosureThreads, sf::mlp::kClosureSmem, S(s)>>>(
-                g, iw, X, tiles, fallback, (double *)Akv, (double *)Akt, err);
+        e = sf::launch_dep(c, relu ? k_closure_mlp<double, kActRelu> : k_closure_mlp<double, kActGelu>, grid,
+                           sf::mlp::kClosureThreads, sf::mlp::kClosureSmem, S(s), g, iw, X, tiles, fallback,
+                           (double *)Akv, (double *)Akt, err);
     } else {
         auto g = sf::Ops<float>::geo(c);
         sf::mlp::k_closure_rows<float><<<nblk(nrows, 128), 128, 0, S(s)>>>(
             g, (const float *)u, (const float *)v, (const float *)z_r, (const float *)bvf,
             (const float *)sustr, (const float *)svstr, nfeat, lo, hi, fallback, fallback_list,
             fallback_count, X, nrows);
-        (relu ? k_closure_mlp<float, kActRelu> : k_closure_mlp<float, kActGelu>)
-            <<<grid, sf::mlp::kClosureThreads, sf::mlp::kClosureSmem, S(s)>>>(
-                g, iw, X, tiles, fallback, (float *)Akv, (float *)Akt, err);
+        e = sf::launch_dep(c, relu ? k_closure_mlp<float, kActRelu> : k_closure_mlp<float, kActGelu>, grid,
+                           sf::mlp::kClosureThreads, sf::mlp::kClosureSmem, S(s), g, iw, X, tiles, fallback,
+                           (float *)Akv, (float *)Akt, err);
     }
-    e = cudaGetLastError();
+    const cudaError_t el = cudaGetLastError();
+    if (e == cudaSuccess) e = el;
     return e == cudaSuccess ? SF_OK : mcuda(e, "sf_closure_step");
 }
 
