@@ -309,6 +309,10 @@ __global__ void __launch_bounds__(256) k_mse(long n, int nvalid, const float *__
 __global__ void k_adam(long n, float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
                        float *__restrict__ v, __nv_bfloat16 *__restrict__ wb, float lr, float b1,
                        float b2, float c1, float c2, float eps) {
+    // A step's ten updates are small launches after one another: the next one's blocks may come in at once
+    // and wait there.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     const float gg = g[e];
@@ -1498,9 +1502,19 @@ int sf_mlp_adam(long n, float *w, const float *g, float *m, float *v, void *w_bf
                 float b1, float b2, int step, float eps, sf_stream s) {
     if (n <= 0 || !w || !g || !m || !v || step < 1) return mfail(SF_EINVAL, "bad argument");
     const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-    sf::mlp::k_adam<<<nblk(n, 256), 256, 0, S(s)>>>(n, w, g, m, v, (__nv_bfloat16 *)w_bf16, lr, b1, b2,
-                                                     c1, c2, eps);
-    cudaError_t e = cudaGetLastError();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = nblk(n, 256);
+    cfg.blockDim = 256;
+    cfg.stream = S(s);
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, sf::mlp::k_adam, n, w, g, m, v, (__nv_bfloat16 *)w_bf16, lr, b1, b2, c1, c2,
+                                       eps);
+    const cudaError_t el = cudaGetLastError();
+    if (e == cudaSuccess) e = el;
     return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_adam");
 }
 
