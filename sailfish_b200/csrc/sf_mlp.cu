@@ -272,14 +272,16 @@ __global__ void k_colsum(long n, const float *__restrict__ G, float *__restrict_
 
 // MSE on the first nvalid outputs: dY = 2 (Y - T) / (n * nvalid), loss accumulated into *loss: sums of
 // a thread's elements, then of its block, one atomic per block (at most kMseBlocks of them: each
-// rounds the loss once; an atomic per warp rounded it n * 4 times and serialised in L2).
+// rounds the loss once; an atomic per warp rounded it n * 4 times and serialised in L2).  Error of the
+// FP32 sum at 3056 to 12000 rows: up to 4e-6 with an atomic per warp, 3.5e-7 now.
 // VEC: four elements at a time (buffers on 16-byte boundaries).
-constexpr int kMseBlocks = 592;
+constexpr int kMseBlocks = 148, kMseThreads = 1024;
 template <bool VEC>
-__global__ void __launch_bounds__(256) k_mse(long n, int nvalid, const float *__restrict__ Y,
+__global__ void __launch_bounds__(kMseThreads) k_mse(long n, int nvalid, const float *__restrict__ Y,
                                              const float *__restrict__ T, float *__restrict__ dY, float *loss) {
     constexpr int E = VEC ? 4 : 1;
     using V = std::conditional_t<VEC, float4, float>;
+    pdl_enter();
     float l = 0.f;
     const float scale = (float)(n * nvalid);
 #pragma unroll 2
@@ -296,12 +298,13 @@ __global__ void __launch_bounds__(256) k_mse(long n, int nvalid, const float *__
         reinterpret_cast<V *>(dY)[e] = g;
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    __shared__ float part[8];
+    __shared__ float part[kMseThreads / 32];
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = l;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) l += part[w];
-        if (l != 0.f) atomicAdd(loss, l);
+    if (threadIdx.x < 32) {
+        l = part[threadIdx.x];
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+        if (threadIdx.x == 0 && l != 0.f) atomicAdd(loss, l);
     }
 }
 
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_infer(InferW w, long n,
 // operand lives in L2 (about 60 MB with the saved activations), so the passes are bound by the
 // chain product -> epilogue -> product of a tile and by each SM's L1 path, not by HBM or the tensor
 // cores (7.5 GFLOP, 5 us).  Layer by layer through k_gemm an optimizer step of 8192 rows took 15.3 ms
-// (each dW product sums all its rows in one CTA, staged element by element); now 0.215 ms: k_fwd
+// (each dW product sums all its rows in one CTA, staged element by element); now 0.188 ms: k_fwd
 // 36 us, k_bwd_rows 20, k_bwd_dw 96, the rest the loss and Adam launches.
 //   k_fwd      one CTA per 128-row tile: the five layers in a row, the next layer's weights loaded
 //              beside the current product, writing the pre-activations and activations the
@@ -636,6 +639,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_fwd(InferW w, long n, cons
     float *turn = reinterpret_cast<float *>(sW + 2 * kPTile) + warp * 32 * kTurn;
     const long r0 = (long)blockIdx.x * kTile + rb;
     const int rows = (int)(n - r0 < 32 ? n - r0 : 32);
+    pdl_enter();
     if (warp == 0) tmem_alloc(&tmem_base);
     if (tid == 0) {
         mbar_init(&mbar);
@@ -702,7 +706,10 @@ struct BwdPtrs {
     float *dW[SF_MLP_LAYERS], *db[SF_MLP_LAYERS];
 };
 
-__global__ void k_zero_db(BwdPtrs d) { d.db[blockIdx.x][threadIdx.x] = 0.f; }
+__global__ void k_zero_db(BwdPtrs d) {
+    pdl_enter();
+    d.db[blockIdx.x][threadIdx.x] = 0.f;
+}
 
 // A CTA takes the rows whose index modulo 256 is 4 blockIdx .. 4 blockIdx + 3, one residue for each 32
 // tile rows (32 rows 256 apart), so that db is added up as k_colsum does: one sequential FP32 sum per
@@ -721,6 +728,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_bwd_rows(InferW w, long n,
     float *turn = reinterpret_cast<float *>(sW + 2 * kPTile) + warp * 32 * kTurn;
     const int res0 = blockIdx.x * 4, res = res0 + (warp & 3);
     constexpr long kPitch = (long)kDbParts * kTile;   // from a row to the next of its residue
+    pdl_enter();
     if (warp == 0) tmem_alloc(&tmem_base);
     if (tid == 0) {
         mbar_init(&mbar);
@@ -914,6 +922,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
              const float *__restrict__ dY, const __nv_bfloat16 *__restrict__ Gb, BwdPtrs d, int *err) {
     const int c0 = blockIdx.x * kDwCols, l = blockIdx.y;
     const float *Xl = l == 0 ? X : acts + (long)(l - 1) * n * kTile;
+    pdl_enter();
     if (l == SF_MLP_LAYERS - 1) bwd_dw<true>(n, Xl, dY, nullptr, c0, d.dW[l], err);
     else bwd_dw<false>(n, Xl, nullptr, Gb + (long)l * n * kTile, c0, d.dW[l], err);
 }
@@ -1351,6 +1360,25 @@ bool grads_ok(float *const *dW, float *const *db) {
     return true;
 }
 
+// A training kernel as a dependent launch: it waits for its predecessor itself (griddepcontrol.wait).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_train(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                         Args... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    const cudaError_t el = cudaGetLastError();
+    return e == cudaSuccess ? el : e;
+}
+
 // The raised shared-memory limits are per-device function attributes: set once on each device.
 int train_attrs() {
     static bool done[64] = {};
@@ -1410,9 +1438,8 @@ int sf_mlp_forward(const sf_mlp_params *w, int n, const float *X, float *Y, floa
         int rc = train_attrs();
         if (rc) return rc;
         auto k = w->act == SF_MLP_RELU ? sf::mlp::k_fwd<sf::mlp::kActRelu> : sf::mlp::k_fwd<sf::mlp::kActGelu>;
-        k<<<nblk(n, kTile), sf::mlp::kTrainThreads, sf::mlp::kRowsSmem, S(s)>>>(infer_w(w), n, X, Y, acts,
-                                                                               pre, err);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_train(k, nblk(n, kTile), sf::mlp::kTrainThreads, sf::mlp::kRowsSmem, S(s),
+                                           infer_w(w), n, X, Y, acts, pre, err);
         return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_forward");
     }
     const long ld = kTile;
@@ -1445,14 +1472,16 @@ int sf_mlp_backward(const sf_mlp_params *w, int n, const float *X, const float *
             d.db[l] = db[l];
         }
         auto *Gb = reinterpret_cast<__nv_bfloat16 *>(work);   // 4 layers x n x 128 BF16: all of it
-        sf::mlp::k_zero_db<<<SF_MLP_LAYERS, kTile, 0, S(s)>>>(d);
         auto k = w->act == SF_MLP_RELU ? sf::mlp::k_bwd_rows<sf::mlp::kActRelu>
                                        : sf::mlp::k_bwd_rows<sf::mlp::kActGelu>;
-        k<<<sf::mlp::kDbParts / 4, sf::mlp::kTrainThreads, sf::mlp::kRowsSmem, S(s)>>>(infer_w(w), n, pre, dY, d,
-                                                                                      Gb, err);
-        sf::mlp::k_bwd_dw<<<dim3(kTile / sf::mlp::kDwCols, SF_MLP_LAYERS),
-                            sf::mlp::kTrainThreads, sf::mlp::kDwSmem, S(s)>>>(n, X, acts, dY, Gb, d, err);
-        const cudaError_t e = cudaGetLastError();
+        // each is a dependent launch: an optimizer step of 8192 rows 197 us with plain ones, 188 now
+        cudaError_t e = launch_train(sf::mlp::k_zero_db, SF_MLP_LAYERS, kTile, 0, S(s), d);
+        if (e == cudaSuccess)
+            e = launch_train(k, sf::mlp::kDbParts / 4, sf::mlp::kTrainThreads, sf::mlp::kRowsSmem, S(s), infer_w(w),
+                             n, pre, dY, d, Gb, err);
+        if (e == cudaSuccess)
+            e = launch_train(sf::mlp::k_bwd_dw, dim3(kTile / sf::mlp::kDwCols, SF_MLP_LAYERS),
+                             sf::mlp::kTrainThreads, sf::mlp::kDwSmem, S(s), n, X, acts, dY, Gb, d, err);
         return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_backward");
     }
     const long ld = kTile;
@@ -1491,10 +1520,10 @@ int sf_mlp_backward(const sf_mlp_params *w, int n, const float *X, const float *
 int sf_mlp_mse(int n, int nvalid, const float *Y, const float *T, float *dY, float *loss, sf_stream s) {
     if (n <= 0 || !Y || !T || !dY || !loss) return mfail(SF_EINVAL, "bad argument");
     const bool vec = aligned16(Y) && aligned16(T) && aligned16(dY);
-    const unsigned nb = nblk((long)n * kTile / (vec ? 4 : 1), 256);
-    (vec ? sf::mlp::k_mse<true> : sf::mlp::k_mse<false>)<<<nb < sf::mlp::kMseBlocks ? nb : sf::mlp::kMseBlocks, 256, 0,
-                                                           S(s)>>>(n, nvalid, Y, T, dY, loss);
-    cudaError_t e = cudaGetLastError();
+    const unsigned nb = nblk((long)n * kTile / (vec ? 4 : 1), sf::mlp::kMseThreads);
+    const cudaError_t e = launch_train(vec ? sf::mlp::k_mse<true> : sf::mlp::k_mse<false>,
+                                       nb < sf::mlp::kMseBlocks ? nb : sf::mlp::kMseBlocks,
+                                       sf::mlp::kMseThreads, 0, S(s), n, nvalid, Y, T, dY, loss);
     return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_mse");
 }
 
@@ -1502,19 +1531,8 @@ int sf_mlp_adam(long n, float *w, const float *g, float *m, float *v, void *w_bf
                 float b1, float b2, int step, float eps, sf_stream s) {
     if (n <= 0 || !w || !g || !m || !v || step < 1) return mfail(SF_EINVAL, "bad argument");
     const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = nblk(n, 256);
-    cfg.blockDim = 256;
-    cfg.stream = S(s);
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, sf::mlp::k_adam, n, w, g, m, v, (__nv_bfloat16 *)w_bf16, lr, b1, b2, c1, c2,
-                                       eps);
-    const cudaError_t el = cudaGetLastError();
-    if (e == cudaSuccess) e = el;
+    const cudaError_t e = launch_train(sf::mlp::k_adam, nblk(n, 256), 256, 0, S(s), n, w, g, m, v,
+                                       (__nv_bfloat16 *)w_bf16, lr, b1, b2, c1, c2, eps);
     return e == cudaSuccess ? SF_OK : mcuda(e, "sf_mlp_adam");
 }
 
