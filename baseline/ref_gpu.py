@@ -62,7 +62,7 @@ def generate(verbose=False):
     """Build recipe: the reference's kernel sources, renamed as its loader renames them, into
     baseline/_ref/src.  Returns False where the reference checkout is absent."""
     ref = reference_root()
-    if not os.path.isdir(ref):
+    if not os.path.isfile(os.path.join(ref, "modules", "mod_cppkernels.h")):
         return False
     os.makedirs(SRC, exist_ok=True)
     with open(os.path.join(ref, "modules", "mod_cppkernels.h"), encoding="utf-8-sig") as f:

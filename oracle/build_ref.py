@@ -72,7 +72,7 @@ def lib_path(name, suffix=""):
 
 def build(verbose=False, opt="-O2"):
     ref = reference_root()
-    if not os.path.isdir(ref):
+    if not os.path.isfile(os.path.join(ref, "modules", "mod_cppkernels.h")):
         if verbose:
             print("reference not present at %s; oracle/_ref not rebuilt" % ref)
         return False
