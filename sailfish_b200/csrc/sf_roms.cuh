@@ -865,7 +865,9 @@ constexpr int roms_sub_blocks() { return !LATE ? 1 : (sizeof(R) == 4 ? 3 : 2); }
 template <typename R, int H, bool LATE>
 __global__ void __launch_bounds__(32 * H, roms_sub_blocks<R, LATE>()) k_roms_sub(Geo<R> g, RomsArgs<R> a) {
     extern __shared__ __align__(16) unsigned char sub_smem[];
-    roms_sub_tile<R, H, LATE>(g, a, (int)blockIdx.x * kSubCols, (int)blockIdx.y * (H - 3), sub_smem);
+    // grid.z: 65,535 rows of tiles each, past the end no node is owned
+    roms_sub_tile<R, H, LATE>(g, a, (int)blockIdx.x * kSubCols, (int)(blockIdx.z * gridDim.y + blockIdx.y) * (H - 3),
+                              sub_smem);
 }
 template <typename R, int H, bool LATE>
 __global__ void __launch_bounds__(32 * H, roms_sub_blocks<R, LATE>()) kb_roms_sub(const Member<R> *mt, const int2 *bm,
@@ -980,18 +982,26 @@ __global__ void __launch_bounds__(256) kb_roms_walls3d(const Member<R> *mt, cons
     roms_walls3d_at(m.g, u + m.o3, v + m.o3, m.p);
 }
 
+constexpr int kGridY = 65535;   // blocks a grid holds along y
+// Rows a warp walks: at least as many as a grid of kRomsWarps warps a block needs for J rows.
+inline int roms_fit_rows(int rows, int J) {
+    const int least = (int)(((long)J + (long)kGridY * kRomsWarps - 1) / ((long)kGridY * kRomsWarps));
+    return rows > least ? rows : least;
+}
+
 template <typename R>
 cudaError_t Ops<R>::roms_phase(const sf_ctx *c, const RomsArgs<R> &a, cudaStream_t s) {
     const int B = 32 * kRomsWarps;
     if (a.phase == 3) {
-        dim3 grid((c->I + kSubCols - 1) / kSubCols, (c->J + kSubRows - 4) / (kSubRows - 3));
+        const int ny = (c->J + kSubRows - 4) / (kSubRows - 3);
+        dim3 grid((c->I + kSubCols - 1) / kSubCols, ny < kGridY ? ny : kGridY, (ny + kGridY - 1) / kGridY);
         if (c->nmem > 1) grid = dim3(c->nbm_sub);
         // few tiles: one node's latency counts, everything in registers (514 x 258 nodes, 580 tiles, FP32:
         // 367 us a loop of 52 substeps against 437; 130 x 66, FP64: 220 against 229); many: blocks per
         // SM count (642 x 322, 864 tiles, FP32: 480 against 512; 514 x 258, FP64: 638 against 716; at
         // 258 x 130, 150 tiles, FP64 takes 333 and 336)
-        return (long)grid.x * grid.y >= (sizeof(R) == 4 ? 720 : 200) ? roms_sub_launch<R, true>(c, a, grid, s)
-                                                                     : roms_sub_launch<R, false>(c, a, grid, s);
+        return (long)grid.x * grid.y * grid.z >= (sizeof(R) == 4 ? 720 : 200) ? roms_sub_launch<R, true>(c, a, grid, s)
+                                                                              : roms_sub_launch<R, false>(c, a, grid, s);
     }
     if (c->nmem > 1) {
         if (a.phase == 2)
@@ -1000,7 +1010,7 @@ cudaError_t Ops<R>::roms_phase(const sf_ctx *c, const RomsArgs<R> &a, cudaStream
         return launch_dep(c, k, c->nbm_roms, B, 0, s, mt<R>(c), c->bm_roms, a, c->roms_rows);
     }
     if (a.phase == 2) return launch_dep(c, k_roms_acc<R>, blocks_for(c->s2, 256), 256, 0, s, geo(c), a);
-    const int rows = c->roms_rows;
+    const int rows = roms_fit_rows(c->roms_rows, c->J);
     const dim3 grid((c->I + kRomsCols - 1) / kRomsCols, (c->J + rows * kRomsWarps - 1) / (rows * kRomsWarps));
     auto k = a.phase == 0 ? k_roms_phase<R, 0> : k_roms_phase<R, 1>;
     return launch_dep(c, k, grid, B, 0, s, geo(c), a, rows);
@@ -1026,7 +1036,7 @@ cudaError_t Ops<R>::roms_rhs3d(const sf_ctx *c, const R *u, const R *v, const R 
     } else {
         // rows a warp walks: 8 (1026 x 514 x 50 in FP32: 4, 8, 16, 32, 64 rows 0.177, 0.158, 0.162, 0.168,
         // 0.184 ms), 32 on large grids (2050 x 1026 x 50: 0.685, 0.618, 0.627, 0.605, 0.584)
-        const int rows = c->s2 >= (1L << 20) ? 32 : 8;
+        const int rows = roms_fit_rows(c->s2 >= (1L << 20) ? 32 : 8, c->J);
         const dim3 grid((c->I + kRomsCols - 1) / kRomsCols, (c->J + rows * kRomsWarps - 1) / (rows * kRomsWarps),
                         c->N + 1);
         k_roms_rhs3d<R><<<grid, B, 0, s>>>(geo(c), u, v, Huon, Hvom, Hz, ru, rv, rows);
