@@ -291,9 +291,9 @@ __global__ void __launch_bounds__(kMseThreads) k_mse(long n, int nvalid, const f
 #pragma unroll
         for (int q = 0; q < E; ++q) {
             const bool in = (int)(e % (kTile / E)) * E + q < nvalid;
-            const float d = in ? reinterpret_cast<const float *>(&y)[q] - reinterpret_cast<const float *>(&t)[q] : 0.f;
-            reinterpret_cast<float *>(&g)[q] = 2.f * d / scale;
-            l += d * d / scale;
+            const float d = reinterpret_cast<const float *>(&y)[q] - reinterpret_cast<const float *>(&t)[q];
+            reinterpret_cast<float *>(&g)[q] = in ? 2.f * d / scale : 0.f;   // no division without columns (scale 0)
+            l += in ? d * d / scale : 0.f;
         }
         reinterpret_cast<V *>(dY)[e] = g;
     }
