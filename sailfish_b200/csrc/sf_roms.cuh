@@ -621,9 +621,16 @@ struct RomsRhs {
 };
 
 // Levels whose loads the column solve issues together (1003 x 501 x 50, FP32: 2, 4, 6, 8, 12 levels 0.59,
-// 0.59, 0.47, 0.45, 0.53 ms, 118 to 197 registers; FP64 4, 6, 8: 1.29, 1.27, 1.33).
+// 0.59, 0.47, 0.45, 0.53 ms; FP64 4, 6, 8: 1.29, 1.27, 1.33), and the blocks per SM its registers are capped
+// for.  Columns of at most 16 levels (SHORT) have few chunks to issue and little shared memory, so more blocks
+// hide the latency instead: 1026 x 514 x 6 in FP32 112 us with 8 levels and 3 blocks, 79 with 4 and 6, 72 with
+// 2 and 8; FP64 224, 171 and 132 (2 and 10); 16 levels FP32 196, 143, 132, FP64 433, 331, 285; at 24 levels
+// the long form leads (FP32 255 against 282 us).
+constexpr int kRomsShortN = 16;
 template <typename R>
-constexpr int roms_col_chunk() { return sizeof(R) == 4 ? 8 : 6; }
+constexpr int roms_col_chunk(bool SHORT) { return SHORT ? 2 : (sizeof(R) == 4 ? 8 : 6); }
+template <typename R>
+constexpr int roms_col_blocks(bool SHORT) { return !SHORT ? 3 : (sizeof(R) == 4 ? 8 : 10); }
 // A pivot of the elimination as its divisions use it: in FP32 the reciprocal (a / b through
 // __fdividef is a times the hardware reciprocal of b, bit for bit in b's normal range, and every
 // pivot divides twice), in FP64 the pivot itself (IEEE division).
@@ -644,7 +651,7 @@ __device__ __forceinline__ R roms_div(R a, R b) { return over_pivot(a, roms_pivo
 // solution does.  Levels are taken in whole chunks whose loads are issued together, then one by
 // one: a test per level inside a chunk (the level below N?) cost some 300 cycles a level.
 // Off: element offsets in a field (32-bit where they fit).
-template <typename R, int T, typename Off>
+template <typename R, int T, typename Off, bool SHORT>
 __device__ __forceinline__ double roms_column(const Geo<R> &g, const int p, const int d, R *__restrict__ u,
                                               RomsRhs<R> rs, R c0, R c1, R c2, const R *__restrict__ Hz,
                                               const R *__restrict__ Akv, const R *__restrict__ z_r,
@@ -715,7 +722,7 @@ __device__ __forceinline__ double roms_column(const Geo<R> &g, const int p, cons
                       q1[c], q2[c], uo[c]);
         }
     };
-    in_chunks<roms_col_chunk<R>()>(N - 1, levels);
+    in_chunks<roms_col_chunk<R>(SHORT)>(N - 1, levels);
     eliminate(Hz[o], Hz[o - d], R(0), R(0), rs.r0[o], rs.r1[o], rs.r2[o], u[o]);
     // back substitution
     R x = over_pivot(xp, pv);
@@ -761,7 +768,7 @@ constexpr int roms_col_threads() { return sizeof(R) == 4 ? 128 : 64; }
 // i = 1..I-2), one thread per face column: the U column (west face) or the V column (south face,
 // vcol) of rho point p; and the barotropic restart: ubar, vbar in slots n and scratch = the new
 // depth-mean velocities at those faces, 0 elsewhere.
-template <typename R, int T, typename Off>
+template <typename R, int T, typename Off, bool SHORT>
 __device__ __forceinline__ void roms_step3d_at(const Geo<R> &g, R *__restrict__ u,
                                                R *__restrict__ v, RomsRhs<R> ru, RomsRhs<R> rv,
                                                R c0, R c1, R c2, R *__restrict__ ubar_n,
@@ -778,13 +785,13 @@ __device__ __forceinline__ void roms_step3d_at(const Geo<R> &g, R *__restrict__ 
     R bar = R(0);
     if (!vcol) {
         if (i >= 2 && i <= g.I - 2 && j >= 1 && j <= g.J - 2)
-            bar = (R)roms_column<R, T, Off>(g, p, 1, u, ru, c0, c1, c2, Hz, Akv, z_r, W, DU[p], g.on_u[p], dt,
+            bar = (R)roms_column<R, T, Off, SHORT>(g, p, 1, u, ru, c0, c1, c2, Hz, Akv, z_r, W, DU[p], g.on_u[p], dt,
                                        lamdt, col);
         ubar_n[p] = bar;
         ubar_s[p] = bar;
     } else {
         if (j >= 2 && j <= g.J - 2 && i >= 1 && i <= g.I - 2)
-            bar = (R)roms_column<R, T, Off>(g, p, g.I, v, rv, c0, c1, c2, Hz, Akv, z_r, W, DV[p], g.om_v[p],
+            bar = (R)roms_column<R, T, Off, SHORT>(g, p, g.I, v, rv, c0, c1, c2, Hz, Akv, z_r, W, DV[p], g.om_v[p],
                                        dt, lamdt, col);
         vbar_n[p] = bar;
         vbar_s[p] = bar;
@@ -943,19 +950,19 @@ __global__ void __launch_bounds__(256) kb_roms_stress3d(const Member<R> *mt, con
 }
 // A point block's U columns and its V columns are consecutive blocks: Hz, Akv, z_r and W are then read
 // from DRAM once for both.
-template <typename R, typename Off>
-__global__ void __launch_bounds__(roms_col_threads<R>(), 3) k_roms_step3d(
+template <typename R, typename Off, bool SHORT>
+__global__ void __launch_bounds__(roms_col_threads<R>(), roms_col_blocks<R>(SHORT)) k_roms_step3d(
     Geo<R> g, R *u, R *v, RomsRhs<R> ru, RomsRhs<R> rv, R c0, R c1, R c2, R *ubar_n, R *vbar_n, R *ubar_s,
     R *vbar_s, const R *Hz, const R *Akv, const R *z_r, const R *W, const double *DU, const double *DV, R dt,
     R lamdt) {
     constexpr int T = roms_col_threads<R>();
     extern __shared__ __align__(16) unsigned char col_smem[];
-    roms_step3d_at<R, T, Off>(g, u, v, ru, rv, c0, c1, c2, ubar_n, vbar_n, ubar_s, vbar_s, Hz, Akv, z_r, W, DU, DV,
+    roms_step3d_at<R, T, Off, SHORT>(g, u, v, ru, rv, c0, c1, c2, ubar_n, vbar_n, ubar_s, vbar_s, Hz, Akv, z_r, W, DU, DV,
                          dt, lamdt, (long)(blockIdx.x >> 1) * T + threadIdx.x, blockIdx.x & 1,
                          reinterpret_cast<R *>(col_smem) + threadIdx.x);
 }
-template <typename R, typename Off>
-__global__ void __launch_bounds__(roms_col_threads<R>(), 3) kb_roms_step3d(
+template <typename R, typename Off, bool SHORT>
+__global__ void __launch_bounds__(roms_col_threads<R>(), roms_col_blocks<R>(SHORT)) kb_roms_step3d(
     const Member<R> *mt, const int2 *bm, R *u, R *v, RomsRhs<R> ru, RomsRhs<R> rv, R c0, R c1, R c2, R *ubar_n,
     R *vbar_n, R *ubar_s, R *vbar_s, const R *Hz, const R *Akv, const R *z_r, const R *W, const double *DU,
     const double *DV, R dt, R lamdt) {
@@ -966,7 +973,7 @@ __global__ void __launch_bounds__(roms_col_threads<R>(), 3) kb_roms_step3d(
     const int part = (int)(blockIdx.x >> 1) % kPart;
     const long o3 = M.off3, o2 = M.off2;
     const RomsRhs<R> a{ru.r0 + o3, ru.r1 + o3, ru.r2 + o3}, b{rv.r0 + o3, rv.r1 + o3, rv.r2 + o3};
-    roms_step3d_at<R, T, Off>(M.g, u + o3, v + o3, a, b, c0, c1, c2, ubar_n + o2, vbar_n + o2, ubar_s + o2,
+    roms_step3d_at<R, T, Off, SHORT>(M.g, u + o3, v + o3, a, b, c0, c1, c2, ubar_n + o2, vbar_n + o2, ubar_s + o2,
                          vbar_s + o2, Hz + M.offN, Akv + o3, z_r + M.offN, W + o3, DU + o2, DV + o2, dt, lamdt,
                          (long)mb.y * 128 + part * T + threadIdx.x, blockIdx.x & 1,
                          reinterpret_cast<R *>(col_smem) + threadIdx.x);
@@ -1058,9 +1065,9 @@ cudaError_t Ops<R>::roms_step3d(const sf_ctx *c, R *u, R *v, const R *const *ru,
     if (dev < 0 || dev >= 64 || !done[dev]) {
         const auto at = cudaFuncAttributeMaxDynamicSharedMemorySize;
         const int most = 2 * kRomsMaxN * T * (int)sizeof(R);
-        for (auto k : {k_roms_step3d<R, int>, k_roms_step3d<R, long>})
+        for (auto k : {k_roms_step3d<R, int, false>, k_roms_step3d<R, long, false>})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, most);
-        for (auto k : {kb_roms_step3d<R, int>, kb_roms_step3d<R, long>})
+        for (auto k : {kb_roms_step3d<R, int, false>, kb_roms_step3d<R, long, false>})
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, most);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) done[dev] = true;
@@ -1068,12 +1075,15 @@ cudaError_t Ops<R>::roms_step3d(const sf_ctx *c, R *u, R *v, const R *const *ru,
     const int N = c->nmem > 1 ? c->maxN : c->N, smem = 2 * N * T * (int)sizeof(R);
     // 32-bit offsets within a member's field: (N + 2) levels of at most the pool's points
     const bool fits = (long)(N + 2) * c->s2 < (1L << 31);
+    const bool brief = fits && N <= kRomsShortN;   // at most 16 KB of shared memory a block
     if (c->nmem > 1)
-        (fits ? kb_roms_step3d<R, int> : kb_roms_step3d<R, long>)<<<2 * (128 / T) * c->nbm_128, T, smem, s>>>(
+        (brief ? kb_roms_step3d<R, int, true>
+         : fits ? kb_roms_step3d<R, int, false> : kb_roms_step3d<R, long, false>)<<<2 * (128 / T) * c->nbm_128, T, smem, s>>>(
             mt<R>(c), c->bm_128, u, v, a, b, (R)coef[0], (R)coef[1], (R)coef[2], ubar_n, vbar_n, ubar_s, vbar_s,
             Hz, Akv, z_r, W, DU, DV, (R)dt, (R)lamdt);
     else
-        (fits ? k_roms_step3d<R, int> : k_roms_step3d<R, long>)<<<2 * blocks_for(c->s2, T), T, smem, s>>>(
+        (brief ? k_roms_step3d<R, int, true>
+         : fits ? k_roms_step3d<R, int, false> : k_roms_step3d<R, long, false>)<<<2 * blocks_for(c->s2, T), T, smem, s>>>(
             geo(c), u, v, a, b, (R)coef[0], (R)coef[1], (R)coef[2], ubar_n, vbar_n, ubar_s, vbar_s, Hz, Akv, z_r,
             W, DU, DV, (R)dt, (R)lamdt);
     return cudaGetLastError();
