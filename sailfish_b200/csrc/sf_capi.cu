@@ -906,7 +906,7 @@ int sf_ctx_tune(sf_ctx *c, int knob, int value) {
     case SF_TUNE_MO_CHUNK:
         if (value != 0 && value != 4 && value != 5 && value != 8)
             return fail(SF_EINVAL, "chunk is 0, 4, 5 or 8");
-        c->mo_chunk = value;
+        c->mo_chunk = value == 5 ? 4 : value;
         return SF_OK;
     case SF_TUNE_PRED_PAIR:
         if (value < 0 || value > 2) return fail(SF_EINVAL, "pair is 0, 1 or 2");

@@ -137,8 +137,8 @@ struct sf_ctx {
     // by default: on basin4 the column solve took 2.08 ms with it against 1.65 ms with
     // per-element cp.async staging
     int use_bulk = 0;
-    // levels whose loads the fused flux/omega kernel issues together (sf_ctx_tune; 2050 x 1026 x 50 in
-    // FP32: 0.74, 0.76 and 0.86 ms with 4, 5 and 8 at 3 blocks per SM)
+    // levels whose loads the fused flux/omega kernel issues together (sf_ctx_tune; 1026 x 514 x 50:
+    // FP32 234 and 255 us with 4 and 8, FP64 539 and 537)
     int mo_chunk = 4;
     // fused predictor in its paired form (two nodes per thread) where the grid allows it: 1
     // with 16-row blocks, 2 with 8-row blocks (basin4 loop 4.27 and 4.18 ms), 0 scalar (4.49)

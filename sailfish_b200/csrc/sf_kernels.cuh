@@ -1362,8 +1362,8 @@ __device__ __forceinline__ void rhs3d_march_body(const Geo<R> &g, const R *__res
 // ------------------------------------------------------------------------------------------
 // C > 0: levels whose loads the fused flux/omega kernel issues together on its interior
 // columns (sf_ctx_tune knob SF_TUNE_MO_CHUNK); 0: one level at a time, the loop unrolled by 4;
-// -1: omega alone (no fluxes), the fluxes' loads issued 16 levels at a time
-template <typename R, int C = 0>
+// -1: omega alone (no fluxes), 16 levels in a chunk
+template <typename R, int C>
 __device__ __forceinline__ void maxflux_omega_body(
     const Geo<R> &g, const R *__restrict__ u, const R *__restrict__ v, R *Huon, R *Hvom,
     const R *__restrict__ Hz, R *__restrict__ W, const R *__restrict__ z_w, int do_flux,
@@ -1416,8 +1416,9 @@ __device__ __forceinline__ void maxflux_omega_body(
         R Wk = R(0);
         Wc(0) = R(0);
         if (C < 0 && !rc) {
-            // omega alone: the four fluxes of a chunk of kO levels loaded together (basin4:
-            // 0.45 ms with 16, 0.48 with 8, 0.66 one level at a time)
+            // omega alone: the four fluxes of a chunk of levels without a test a level, so that their loads
+            // issue ahead of its arithmetic, as many together as the registers hold (2050 x 1026 x 50 in FP32
+            // one level at a time 0.66 ms, 0.46 with 64 registers)
             long o0 = s2 + p;
             int K0 = 1;
             in_chunks<16>(N - 1, [&](auto n) {
@@ -1501,9 +1502,7 @@ __device__ __forceinline__ void maxflux_omega_body(
         }
         const R Ws = Wk;
         W[p] = R(0);
-        // the correction, z_w loaded kZ levels at a time (one exposed load latency per chunk):
-        // 32 for omega alone, 16 after the fluxes (basin4: 0.45 and 0.82 ms; 32 after the
-        // fluxes takes 1.14 ms)
+        // the correction, z_w in chunks of 32 levels for omega alone, of 16 after the fluxes
         {
             long o0 = s2 + p;
             int K0 = 1;
@@ -2373,19 +2372,19 @@ __global__ void __launch_bounds__(TX *TY) kb_rhs3d(const Member<R> *mt, const in
                                  mb_.y % ntx, mb_.y / ntx);
 }
 
-// Blocks per SM: chunks of 4 levels want 3 (80 registers; with 2 blocks at 128 they take 0.81 ms, with 4 at
-// 64 0.98, on 2050 x 1026 x 50 in FP32, against 0.74), omega alone 4 (FP64 2).
-template <typename R>
-constexpr int mo_blocks(int C) { return C < 0 ? (sizeof(R) == 4 ? 4 : 2) : 3; }
-template <typename R, int C>
-__global__ void __launch_bounds__(kBlock, mo_blocks<R>(C)) k_maxflux_omega(
+// B: blocks per SM that the registers are capped for (rules in Ops::maxflux_omega).  Chunks of 4 levels in FP32
+// want 3 (80 registers; with 2 blocks at 128 they take 0.81 ms, with 4 at 64 0.98, on 2050 x 1026 x 50,
+// against 0.74), of 8 levels 2 (1026 x 514 x 50: 255 us, 279 with 3), one level at a time 4 (514 x 258 x 32:
+// 41 us, 76 with 3).
+template <typename R, int C, int B>
+__global__ void __launch_bounds__(kBlock, B) k_maxflux_omega(
     Geo<R> g, const R *__restrict__ u, const R *__restrict__ v, R *Huon, R *Hvom, const R *__restrict__ Hz, R *__restrict__ W, const R *__restrict__ z_w,
     int do_flux, int do_omega, R *__restrict__ zeta1, R *__restrict__ zeta2, const double *__restrict__ Zt) {
     maxflux_omega_body<R, C>(g, u, v, Huon, Hvom, Hz, W, z_w, do_flux, do_omega, zeta1, zeta2, Zt,
                              (long)tid_flat());
 }
-template <typename R, int C = 0>
-__global__ void __launch_bounds__(kBlock, mo_blocks<R>(C)) kb_maxflux_omega(
+template <typename R, int C, int B>
+__global__ void __launch_bounds__(kBlock, B) kb_maxflux_omega(
     const Member<R> *mt, const int2 *bm, const R *__restrict__ u, const R *__restrict__ v, R *Huon, R *Hvom, const R *__restrict__ Hz,
     R *__restrict__ W, const R *__restrict__ z_w, int do_flux, int do_omega, R *__restrict__ zeta1, R *__restrict__ zeta2, const double *__restrict__ Zt) {
     SF_MEMBER(bm)
@@ -2683,38 +2682,51 @@ template <typename R>
 cudaError_t Ops<R>::maxflux_omega(const sf_ctx *c, const R *u, const R *v, R *Huon, R *Hvom,
                                   const R *Hz, R *W, const R *z_w, int do_flux, int do_omega,
                                   R *zeta1, R *zeta2, const double *Zt, cudaStream_t s) {
-    const size_t smem = do_omega ? sizeof(R) * (size_t)kBlock * (c->nmem > 1 ? c->maxN : c->N) : 0;
+    constexpr bool F = sizeof(R) == 4;
+    const int N = c->nmem > 1 ? c->maxN : c->N;
+    const int nb = c->nmem > 1 ? c->nbm_pt : (int)blocks_for(c->s2, kBlock);
+    const size_t smem = do_omega ? sizeof(R) * (size_t)kBlock * N : 0;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
         const int most = (int)(sizeof(R) * kBlock * kNMax);
-        cudaFuncSetAttribute(k_maxflux_omega<R, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(k_maxflux_omega<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(k_maxflux_omega<R, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(k_maxflux_omega<R, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(k_maxflux_omega<R, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        for (auto k : {kb_maxflux_omega<R, -1>, kb_maxflux_omega<R, 0>, kb_maxflux_omega<R, 4>})
+        for (auto k : {k_maxflux_omega<R, -1, F ? 4 : 2>, k_maxflux_omega<R, -1, F ? 3 : 1>,
+                       k_maxflux_omega<R, 0, F ? 4 : 3>, k_maxflux_omega<R, 0, F ? 4 : 1>,
+                       k_maxflux_omega<R, 4, 3>, k_maxflux_omega<R, 4, F ? 3 : 2>, k_maxflux_omega<R, 8, 2>})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        for (auto k : {kb_maxflux_omega<R, -1, F ? 4 : 2>, kb_maxflux_omega<R, 0, 3>, kb_maxflux_omega<R, 4, 3>,
+                       kb_maxflux_omega<R, 4, F ? 3 : 2>})
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         attr_set[dev] = true;
     }
+    // the chunked forms address with 32-bit element offsets
+    const bool fits = (long)(N + 1) * c->s2 < (1L << 31);
+    // FP64's running integral takes 2 KB of shared memory a level and block: three blocks of the chunked
+    // form's 80 registers are resident up to 37 levels, and on few blocks a third finds no work
+    // (chunks of 4: 514 x 258 x 64 350 us at 80 registers, 274 at 128; 258 x 130 x 32 37.1 and 31.6;
+    // 1026 x 514 x 8 73.9 and 83.0)
+    const bool three = F || (N <= 37 && nb > 2 * 148);
     if (c->nmem > 1) {
-        const bool fits = (long)(c->maxN + 1) * c->s2 < (1L << 31);
-        auto k = !do_flux ? kb_maxflux_omega<R, -1>
-                 : fits && c->mo_chunk ? kb_maxflux_omega<R, 4> : kb_maxflux_omega<R, 0>;
-        k<<<c->nbm_pt, kBlock, smem, s>>>(mt<R>(c), c->bm_pt, u, v, Huon, Hvom, Hz, W, z_w, do_flux, do_omega,
-                                         zeta1, zeta2, Zt);
+        auto k = !do_flux ? kb_maxflux_omega<R, -1, F ? 4 : 2>
+                 : !(fits && c->mo_chunk) ? kb_maxflux_omega<R, 0, 3>
+                 : three ? kb_maxflux_omega<R, 4, 3> : kb_maxflux_omega<R, 4, F ? 3 : 2>;
+        k<<<nb, kBlock, smem, s>>>(mt<R>(c), c->bm_pt, u, v, Huon, Hvom, Hz, W, z_w, do_flux, do_omega, zeta1, zeta2, Zt);
         return cudaGetLastError();
     }
-    // the chunked forms address with 32-bit element offsets
-    const bool fits = (long)(c->N + 1) * c->s2 < (1L << 31);
-    auto k = !do_flux ? k_maxflux_omega<R, -1>
-             : !fits ? k_maxflux_omega<R, 0>
-             : c->mo_chunk == 8 ? k_maxflux_omega<R, 8>
-             : c->mo_chunk == 5 ? k_maxflux_omega<R, 5>
-             : c->mo_chunk == 4 ? k_maxflux_omega<R, 4> : k_maxflux_omega<R, 0>;
-    k<<<blocks_for(c->s2, kBlock), kBlock, smem, s>>>(
-        geo(c), u, v, Huon, Hvom, Hz, W, z_w, do_flux, do_omega, zeta1, zeta2, Zt);
+    // omega alone: FP32 4 blocks of 64 registers up to 48 levels, 3 of 80 above, where shared memory holds no
+    // more (1026 x 514: 32 levels 62 and 68 us, 48 levels 86 and 89, 50 levels 117 and 85, 56 levels 131 and
+    // 100); FP64 2 of 128, above 56 levels uncapped, one being resident (514 x 258 x 64: 88 and 84 us)
+    const bool deep = N > (F ? 48 : 56);
+    // one level at a time, FP64: 80 registers (514 x 258 x 32 106 us, uncapped 152) but where one block is
+    // resident a SM (258 x 130 x 32 29.6 against 26.8; 514 x 258 x 64 338 against 288)
+    const bool one = nb <= 148 || N > 56;
+    auto k = !do_flux ? (deep ? k_maxflux_omega<R, -1, F ? 3 : 1> : k_maxflux_omega<R, -1, F ? 4 : 2>)
+             : !do_omega ? (F ? k_maxflux_omega<R, 4, 3> : k_maxflux_omega<R, 0, F ? 4 : 3>)
+             : !(fits && c->mo_chunk) ? (one ? k_maxflux_omega<R, 0, F ? 4 : 1> : k_maxflux_omega<R, 0, F ? 4 : 3>)
+             : c->mo_chunk == 8 ? k_maxflux_omega<R, 8, 2>
+             : three ? k_maxflux_omega<R, 4, 3> : k_maxflux_omega<R, 4, F ? 3 : 2>;
+    k<<<nb, kBlock, smem, s>>>(geo(c), u, v, Huon, Hvom, Hz, W, z_w, do_flux, do_omega, zeta1, zeta2, Zt);
     return cudaGetLastError();
 }
 template <typename R>
