@@ -241,6 +241,10 @@ int sf_roms_barotropic_loop(sf_ctx *ctx, sf_state2d *s, double *DU_avg2, double 
  * main2d's step (nonlinear/main2d.py:9-88); first selects forward/backward Euler. */
 int sf_roms_step2d(sf_ctx *ctx, sf_state2d *s, const void *sustr, const void *svstr,
                    double rdrag2, double dtfast, int first, sf_stream stream);
+/* Kernel launches of sf_roms_barotropic_loop for nfast substeps on this context: one for each substep that
+ * runs fused, two or four (by the grid's shape) for the others, one for the averages of substep
+ * nfast + 1; SF_EINVAL for what the loop rejects.  No counterpart in the reference. */
+int sf_roms_loop_launches(const sf_ctx *ctx, int nfast);
 /* nsteps such steps in one call (first applies to the first of them), with the results and the final
  * slots of as many sf_roms_step2d calls. */
 int sf_roms_steps2d(sf_ctx *ctx, sf_state2d *s, const void *sustr, const void *svstr,

@@ -73,6 +73,7 @@ SIGNATURES = {
     "sf_roms_barotropic_loop": [_vp, ctypes.POINTER(State2D), _vp, _vp, _vp, _vp, _d, _i, _dp,
                                 _dp, _d, _vp],
     "sf_roms_step2d": [_vp, ctypes.POINTER(State2D), _vp, _vp, _d, _d, _i, _vp],
+    "sf_roms_loop_launches": [_vp, _i],
     "sf_roms_steps2d": [_vp, ctypes.POINTER(State2D), _vp, _vp, _d, _d, _i, _i, _vp],
     "sf_roms_stress3d": [_vp] * 7 + [_d, _vp],
     "sf_roms_rhs3d": [_vp] * 9,

@@ -322,6 +322,12 @@ int roms_rows_for(long points) {
     return points >= (1L << 20) ? 8 : points >= (1L << 18) ? 4 : points >= (1L << 16) ? 2 : 1;
 }
 
+// What the rules between the forms of the barotropic substep count (roms_by_strips, roms_by_tiles).
+void roms_count(sf_ctx *c, long I, long J) {
+    c->roms_strip_rows += (I + sf::kRomsCols - 1) / sf::kRomsCols * J;
+    c->roms_tiles += (I + sf::kSubCols - 1) / sf::kSubCols * ((J + sf::kSubRows - 4) / (sf::kSubRows - 3));
+}
+
 template <typename R>
 int upload_members(sf_ctx *c, const sf_grid_desc *d, int n, const std::vector<long> &off2,
                    const std::vector<long> &off3, const std::vector<long> &offN,
@@ -468,6 +474,7 @@ int sf_ctx_create_ensemble(const sf_grid_desc *d, int n, sf_ctx **out) {
         for (int m = 0; m < n; ++m) {
             const int I = d[m].L + 1, J = d[m].M + 1;
             const long s2 = (long)I * J;
+            roms_count(c, I, J);
             for (long b = 0; b < (s2 + sf::kPointBlock - 1) / sf::kPointBlock; ++b) pt.push_back({m, (int)b});
             for (long b = 0; b < (s2 + 127) / 128; ++b) b128.push_back({m, (int)b});
             for (int v = 0; v < sf::kRhsTiles; ++v) {
@@ -553,6 +560,7 @@ int sf_ctx_create(const sf_grid_desc *d, sf_ctx **out) {
     c->J = d->M + 1;
     c->s2 = (long)c->I * c->J;
     c->roms_rows = roms_rows_for(c->s2);
+    roms_count(c, c->I, c->J);
     c->hc = d->hc;
     c->Vtransform = d->Vtransform;
     // horizontalAdvection is launched with (grsz*GPUMUL, bksz//GPUMUL) = 512*(s2/512 + 1)
@@ -1105,7 +1113,7 @@ void roms_rotate(sf_state2d *st) {
 // in its place (the levels rotate with period 3, the tendencies with 2), and at least one not fused,
 // so that the scratch slot ends with the predicted level: the caller's slots end as from substeps
 // of two launches each.
-int roms_fused(int left) { return left > 0 ? (left - 1) / 6 * 6 : 0; }
+int roms_fused(const sf_ctx *c, int left) { return left > 0 && sf::roms_by_tiles(c) ? (left - 1) / 6 * 6 : 0; }
 
 void roms_swap(sf_state2d *st) {   // n+1 (written over n-1) becomes n, n becomes n-1
     void **arrs[6] = {st->zeta, st->ubar, st->vbar, st->rzeta, st->rubar, st->rvbar};
@@ -1139,7 +1147,7 @@ int sf_roms_barotropic_loop(sf_ctx *c, sf_state2d *st, double *DU_avg2, double *
     if (!DU_avg2 || !DV_avg2 || !st->Zt_avg1 || !st->DU_avg1 || !st->DV_avg1 || !W1 || !W2)
         return fail(SF_EINVAL, "null accumulator or weights");
     if (nfast < 1 || nfast > 254) return fail(SF_EINVAL, "nfast must be in [1, 254]");
-    const int nfused = roms_fused(nfast - 1);
+    const int nfused = roms_fused(c, nfast - 1);
     for (int iif = 1; iif <= nfast + 1; ++iif) {
         // fast-time averages (step2d_LF_AM3.h.py:778-846), ROMS-indexed weights
         const int acc = iif == 1 ? 2 : 1;
@@ -1164,12 +1172,19 @@ int sf_roms_barotropic_loop(sf_ctx *c, sf_state2d *st, double *DU_avg2, double *
     return SF_OK;
 }
 
+int sf_roms_loop_launches(const sf_ctx *c, int nfast) {
+    if (!c) return fail(SF_EINVAL, "null context");
+    if (nfast < 1 || nfast > 254) return fail(SF_EINVAL, "nfast must be in [1, 254]");
+    const int nfused = roms_fused(c, nfast - 1);
+    return nfused + (nfast - nfused) * (sf::roms_by_strips(c) ? 2 : 4) + 1;
+}
+
 int sf_roms_steps2d(sf_ctx *c, sf_state2d *st, const void *sustr, const void *svstr,
                     double rdrag2, double dtfast, int nsteps, int first, sf_stream s) {
     int rc = roms_check(c, st, sustr, svstr);
     if (rc) return rc;
     if (nsteps < 0) return fail(SF_EINVAL, "nsteps must not be negative");
-    const int f0 = first ? 1 : 0, nfused = roms_fused(nsteps - f0);
+    const int f0 = first ? 1 : 0, nfused = roms_fused(c, nsteps - f0);
     for (int k = 0; k < nsteps; ++k) {
         const bool fused = k >= f0 && k - f0 < nfused;
         const int f = k < f0 ? 1 : 0;

@@ -176,6 +176,7 @@ struct sf_ctx {
     int2 *bm_sub = nullptr;      // tiles of the fused substep
     int nbm_sub = 0;
     int roms_rows = 8;           // rows a warp of those phases walks (roms_rows_for)
+    long roms_strip_rows = 0, roms_tiles = 0;   // rows of the phases' strips, the fused substep's tiles, of all members
     int2 *bm_pipe = nullptr;     // 64-point tiles of the pipelined column solve
     int nbm_pipe = 0;
     long tot2 = 0, tot3 = 0, totN = 0;   // pool sizes
@@ -265,6 +266,27 @@ constexpr int kRomsCols = 29, kRomsWarps = 4;
 // Tiles of the fused substep: columns of its own, staged rows (3 more than its own).  Rows measured
 // at 2050 x 1026 in FP32: 8, 12, 16, 24 staged rows 4.82, 4.35, 5.07, 6.61 ms a loop.
 constexpr int kSubCols = 27, kSubRows = 12;
+
+// Whether the phases go by strips (two launches a substep), else a point a thread (four).  By strips a row of
+// one costs its 32 lanes whether 29 columns exist or one: about 1.3 ns in FP32 on large grids, 4 in FP64, whose
+// 140 to 180 registers leave 8 warps a SM; by points a node costs 0.06 ns (FP64 0.1) and a substep 13 us at least.
+// us a substep in FP32, strips and points: 29 x 3000 10 and 14, 5 x 9000 19 and 13, 17 x 29411 39 and 33, 20 x 25000 32
+// and 33, 33 x 15151 41 and 33, 1026 x 514 25 and 33, 2050 x 1026 100 and 163; FP64: 17 x 1764 12 and 14, 258 x 130
+// 11 and 14, 29 x 3000 18 and 16, 702 x 402 43 and 29, 1026 x 514 72 and 54, 2050 x 1026 264 and 223.
+inline bool roms_by_strips(const sf_ctx *c) {
+    const long rows = c->roms_strip_rows, pts = c->s2;
+    if (c->prec == SF_FP32) return rows <= 6000 || pts >= 20 * rows;
+    return rows <= 1800;
+}
+// Whether runs of leapfrog substeps go fused: about 13 ns a tile of up to 243 nodes in FP32, 27 in FP64, against the
+// phases' times and the averages.  ms a loop of 28 substeps in FP32, tiles and the phases' better form: 5 x 6000
+// 0.31 and 0.39, 16 x 31250 1.23 and 1.10, 20 x 25000 0.94 and 1.09, 28 x 17857 1.36 and 0.84, 1026 x 514 0.66 and 0.85; FP64:
+// 5 x 6000 0.64 and 0.40, 24 x 20833 1.82 and 1.71 (1.69 with the remainders by points), 40 x 12500 2.17 and 1.70, 1026 x 514
+// 1.66 and 1.82, 2050 x 1026 6.0 and 7.3.
+inline bool roms_by_tiles(const sf_ctx *c) {
+    const long tiles = c->roms_tiles, pts = c->s2;
+    return c->prec == SF_FP32 ? 200 * tiles <= pts + 190000 : 225 * tiles <= pts + 100000;
+}
 
 // Launchers, one explicit instantiation per precision (FP64 in a translation unit built
 // without FMA contraction, so that it reproduces the reference's IEEE evaluation).

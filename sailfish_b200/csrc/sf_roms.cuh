@@ -12,12 +12,13 @@
 // ubar(p) on the west face of rho p, vbar(p) on its south face; interior rho i = 1..I-2,
 // j = 1..J-2; interior U faces i = 2..I-2 (walls i = 1, I-1), V faces j = 2..J-2.
 //
-// A substep is two launches: the predictor (free surface, then momentum) and the corrector, each by
-// warps that walk up the rows of a strip of columns (roms_phase_rows).  Time levels: slots b
-// (n-1), n and p (the predicted n+1*); the corrector writes n+1 into b and the host swaps b and
-// n.  Every expression keeps the operand order of the oracle's restatement
-// (oracle/roms_oracle.py), so the FP64 build (no FMA contraction) reproduces it bit for bit; the
-// fast-time averages are FP64 in both precisions.
+// A substep has a predictor and a corrector, each the free surface, then the momentum.  Its forms, of the
+// same bits: in one launch on tiles (roms_sub_tile); in two, a phase each, by warps that walk up the rows
+// of a strip of columns (roms_phase_rows); in four, a point a thread (roms_zeta_point, roms_mom_point).
+// Time levels: slots b (n-1), n and p (the predicted n+1*); the phases' corrector writes n+1 into b and
+// the host swaps b and n (the tiles' levels: roms_sub_tile).  Every expression keeps the operand
+// order of the oracle's restatement (oracle/roms_oracle.py), so the FP64 build (no FMA contraction)
+// reproduces it bit for bit; the fast-time averages are FP64 in both precisions.
 #pragma once
 
 namespace sf {
@@ -273,17 +274,143 @@ __device__ __forceinline__ void roms_phase_rows(const Geo<R> &g, const RomsArgs<
     }
 }
 
-// A whole leapfrog / AM3 substep (predictor and corrector, free surface and momentum) in one launch.
-// A block of 32 x H threads stages 32 columns (27 of them its own: lanes 3..29) and H rows (H - 3 its
-// own: warps 2 .. H - 2), one node per thread.  Every node's inputs are loaded at once; the four
-// stages then follow with x-neighbours by shuffle, y-neighbours through shared memory and three
-// barriers, the halo nodes computing again what their owners compute.  Per substep and node 172
-// bytes in FP32 (levels n and n-1, metrics, stresses and tendencies read once, level n+1 and the
-// tendencies written, 80 bytes of FP64 averages) against 252 in two launches, and one launch
-// latency, which is what small grids pay for.
+// One phase of a substep, a point a thread, in two launches: the free surface (with the averages), then the
+// momentum, which reads the new free surface.  Every thread loads its neighbours' values and forms their
+// fluxes again, but no lane is without a node: strips and tiles hold 29 and 27 columns in 32 lanes, and a basin
+// of a few columns (or a few past a strip) leaves most of them idle.  Where it is the faster one:
+// roms_by_strips, roms_by_tiles.
 //
-// Level n+1 goes to the scratch slot (zout, uout, vout = slot p), because other blocks still read
-// slot b at their halos; the host rotates the three slots.
+// The five averages of a node, A as read (acc 1), with the substep's terms: the predictor's (level n: zeta zk,
+// face transports dun, dvn), then the corrector's (dup, dvp).
+template <typename R>
+__device__ __forceinline__ void roms_averages(const RomsArgs<R> &a, const int p, const double *A, const R zk,
+                                              const double dun, const double dvn, const double dup, const double dvp) {
+    double B[5];
+    if (a.acc == 2) {
+        B[0] = 0.0;
+        B[1] = 0.0;
+        B[2] = 0.0;
+        B[3] = __dmul_rn(a.c2, dun);
+        B[4] = __dmul_rn(a.c2, dvn);
+    } else {
+        B[0] = rsum<R>(A[0], a.c1, (double)zk);
+        B[1] = rsum<R>(A[1], a.c1, dun);
+        B[2] = rsum<R>(A[2], a.c1, dvn);
+        B[3] = rsum<R>(A[3], a.c2, dun);
+        B[4] = rsum<R>(A[4], a.c2, dvn);
+    }
+    a.Zt[p] = B[0];
+    a.DU1[p] = B[1];
+    a.DV1[p] = B[2];
+    a.DU2[p] = rsum<R>(B[3], a.c2c, dup);
+    a.DV2[p] = rsum<R>(B[4], a.c2c, dvp);
+}
+
+// The new free surface of interior node p (i, j), also into the ring nodes next to it.
+template <typename R>
+__device__ __forceinline__ void roms_zeta_out(const Geo<R> &g, R *zout, const int p, const int i, const int j, const R z) {
+    const int I = g.I, J = g.J;
+    const int di = i == 1 ? -1 : (i == I - 2 ? 1 : 0), dj = j == 1 ? -I : (j == J - 2 ? I : 0);
+    zout[p] = z;
+    if (di) zout[p + di] = z;
+    if (dj) zout[p + dj] = z;
+    if (di && dj) zout[p + di + dj] = z;
+}
+
+template <typename R>
+__device__ __forceinline__ R roms_ubar_D(const Geo<R> &g, const R *z, const R *u, const int p) {   // per on_u
+    return rmul(u[p], rmul(R(0.5), (z[p] + g.h[p]) + (z[p - 1] + g.h[p - 1])));
+}
+template <typename R>
+__device__ __forceinline__ R roms_dvom(const Geo<R> &g, const R *z, const R *v, const int p) {
+    return rmul(rmul(v[p], rmul(R(0.5), (z[p] + g.h[p]) + (z[p - g.I] + g.h[p - g.I]))), g.om_v[p]);
+}
+template <typename R, int PH>
+__device__ __forceinline__ void roms_zeta_point(const Geo<R> &g, const RomsArgs<R> &a, const long pl) {
+    if (pl >= g.s2) return;
+    const int p = (int)pl, j = fdiv(p, g.dI), i = p - j * g.I;
+    const bool in = i >= 1 && i <= g.I - 2 && j >= 1 && j <= g.J - 2;
+    const R du = i < 1 ? R(0) : rmul(roms_ubar_D(g, a.zrhs, a.urhs, p), g.on_u[p]);
+    const R dv = j < 1 ? R(0) : roms_dvom(g, a.zrhs, a.vrhs, p);
+    if (in) {
+        const R rz = rfma(-roms_ubar_D(g, a.zrhs, a.urhs, p + 1), g.on_u[p + 1], du) +
+                     (dv - roms_dvom(g, a.zrhs, a.vrhs, p + g.I));
+        R f = rz;
+        if (PH == 0) a.rz_n[p] = rz;
+        else if (!a.first) f = roms_am3(rz, a.rz_n[p], a.rz_b[p]);
+        const R dtz = PH == 0 && !a.first ? (R)(2.0 * a.dtfast) : (R)a.dtfast;
+        roms_zeta_out(g, a.zout, p, i, j, rfma(rmul(rmul(g.pm[p], g.pn[p]), dtz), f, a.zkstp[p]));
+    } else if (PH == 0) {
+        a.rz_n[p] = R(0);
+    }
+    if (PH == 1 && a.acc) {   // level n is the corrector's old level
+        double A[5] = {};
+        if (a.acc == 1) {
+            A[0] = a.Zt[p];
+            A[1] = a.DU1[p];
+            A[2] = a.DV1[p];
+            A[3] = a.DU2[p];
+            A[4] = a.DV2[p];
+        }
+        const R dun = i < 1 ? R(0) : rmul(roms_ubar_D(g, a.zkstp, a.ukstp, p), g.on_u[p]);
+        const R dvn = j < 1 ? R(0) : roms_dvom(g, a.zkstp, a.vkstp, p);
+        roms_averages(a, p, A, a.zkstp[p], (double)dun, (double)dvn, (double)du, (double)dv);
+    }
+}
+// The pressure-gradient surface of a phase at node q, znew its new free surface.
+template <typename R, int PH>
+__device__ __forceinline__ R roms_gp(const RomsArgs<R> &a, const int q, const R znew) {
+    if (a.first) return rmul(R(0.5), a.zkstp[q] + znew);
+    if (PH == 0) return rfma(R(0.68), a.zrhs[q], rmul(R(0.16), a.zkstp[q] + znew));
+    return rfma(R(0.6), znew, rmul(R(0.4), a.zrhs[q]));
+}
+template <typename R, int PH>
+__device__ __forceinline__ void roms_mom_point(const Geo<R> &g, const RomsArgs<R> &a, const long pl) {
+    if (pl >= g.s2) return;
+    const int p = (int)pl, I = g.I, j = fdiv(p, g.dI), i = p - j * I;
+    const bool ri = i >= 1 && i <= I - 2, rj = j >= 1 && j <= g.J - 2;
+    const R *h = g.h, *u = a.urhs, *v = a.vrhs;
+    const R rdrag2 = (R)a.rdrag2, cdt = PH == 0 && !a.first ? (R)a.dtfast : (R)(0.5 * a.dtfast);
+    R unew = R(0), runew = R(0), vnew = R(0), rvnew = R(0);
+    if (ri && rj && (i >= 2 || j >= 2)) {
+        const R zo = a.zout[p], gp = roms_gp<R, PH>(a, p, zo);
+        const R fa = rmul(rmul(R(0.5), a.zrhs[p] + h[p]), g.fomn[p]);
+        const R dk = a.zkstp[p] + h[p], dz = zo + h[p], ue = u[p + 1], vn = v[p + I];
+        if (i >= 2) {
+            const int w = p - 1;
+            const R zw = a.zout[w], fw = rmul(rmul(R(0.5), a.zrhs[w] + h[w]), g.fomn[w]);
+            const R cor = rfma(fa, v[p] + vn, rmul(fw, v[w] + v[w + I]));
+            const R pmn2 = rmul(g.pm[p] + g.pm[w], g.pn[p] + g.pn[w]);
+            const R v4 = rmul(R(0.25), ((v[p] + vn) + v[w]) + v[w + I]);
+            const R ru = roms_rhs<R, false>(g.on_u[p], roms_gp<R, PH>(a, w, zw), gp, h[w], h[p], cor, u[p], v4, rdrag2,
+                                            a.sustr[p], ddiv(R(4.0), pmn2));
+            R f = ru;
+            if (PH == 0) runew = ru;
+            else if (!a.first) f = roms_am3(ru, a.ru_n[p], a.ru_b[p]);
+            unew = roms_new(a.ukstp[p], dk + (a.zkstp[w] + h[w]), pmn2, cdt, f, dz + (zw + h[w]));
+        }
+        if (j >= 2) {
+            const int q = p - I;
+            const R zs = a.zout[q], fs = rmul(rmul(R(0.5), a.zrhs[q] + h[q]), g.fomn[q]);
+            const R cor = rfma(fa, u[p] + ue, rmul(fs, u[q] + u[q + 1]));
+            const R pmn2 = rmul(g.pm[p] + g.pm[q], g.pn[p] + g.pn[q]);
+            const R u4 = rmul(R(0.25), ((u[p] + ue) + u[q]) + u[q + 1]);
+            const R rv = roms_rhs<R, true>(g.om_v[p], roms_gp<R, PH>(a, q, zs), gp, h[q], h[p], cor, v[p], u4, rdrag2,
+                                           a.svstr[p], ddiv(R(4.0), pmn2));
+            R f = rv;
+            if (PH == 0) rvnew = rv;
+            else if (!a.first) f = roms_am3(rv, a.rv_n[p], a.rv_b[p]);
+            vnew = roms_new(a.vkstp[p], dk + (a.zkstp[q] + h[q]), pmn2, cdt, f, dz + (zs + h[q]));
+        }
+    }
+    a.uout[p] = unew;
+    a.vout[p] = vnew;
+    if (PH == 0) {
+        a.ru_n[p] = runew;
+        a.rv_n[p] = rvnew;
+    }
+}
+
 // A copy of one value of the thread's own into its own shared-memory word: in flight without
 // holding a register until it is read (after cp_own_wait).
 template <typename T>
@@ -298,6 +425,17 @@ __device__ __forceinline__ void cp_own_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
+// A whole leapfrog / AM3 substep (predictor and corrector, free surface and momentum) in one launch.
+// A block of 32 x H threads stages 32 columns (27 of them its own: lanes 3..29) and H rows (H - 3 its
+// own: warps 2 .. H - 2), one node per thread.  Every node's inputs are loaded at once; the four
+// stages then follow with x-neighbours by shuffle, y-neighbours through shared memory and three
+// barriers, the halo nodes computing again what their owners compute.  Per substep and node 172
+// bytes in FP32 (levels n and n-1, metrics, stresses and tendencies read once, level n+1 and the
+// tendencies written, 80 bytes of FP64 averages) against 252 in two launches, and one launch
+// latency, which is what small grids pay for.
+//
+// Level n+1 goes to the scratch slot (zout, uout, vout = slot p), because other blocks still read
+// slot b at their halos; the host rotates the three slots.
 template <typename R, int H, bool LATE>
 __device__ __forceinline__ void roms_sub_tile(const Geo<R> &g, const RomsArgs<R> &a, const int i0,
                                               const int j0, unsigned char *raw) {
@@ -859,6 +997,19 @@ __global__ void __launch_bounds__(32 * kRomsWarps) kb_roms_phase(const Member<R>
     roms_phase_rows<R, PH>(M.g, roms_args_at(a, M.off2), bx * kRomsCols,
                            (by * kRomsWarps + (int)(threadIdx.x >> 5)) * nrows, nrows);
 }
+template <typename R, int PH, bool MOM>
+__global__ void __launch_bounds__(256) k_roms_point(Geo<R> g, RomsArgs<R> a) {
+    pdl_enter();
+    if constexpr (MOM) roms_mom_point<R, PH>(g, a, tid_flat());
+    else roms_zeta_point<R, PH>(g, a, tid_flat());
+}
+template <typename R, int PH, bool MOM>
+__global__ void __launch_bounds__(256) kb_roms_point(const Member<R> *mt, const int2 *bm, RomsArgs<R> a) {
+    pdl_enter();
+    const MemberAt<R> m = member_at(mt, bm, 256);
+    if constexpr (MOM) roms_mom_point<R, PH>(m.g, roms_args_at(a, m.o2), m.p);
+    else roms_zeta_point<R, PH>(m.g, roms_args_at(a, m.o2), m.p);
+}
 // Shared memory of a block: per node (LATE) 5 averages and 7 late inputs, 8 exchanged values, and a
 // row of pad on either side of the exchanged fields.
 template <typename R, bool LATE>
@@ -1009,6 +1160,22 @@ cudaError_t Ops<R>::roms_phase(const sf_ctx *c, const RomsArgs<R> &a, cudaStream
         // 258 x 130, 150 tiles, FP64 takes 333 and 336)
         return (long)grid.x * grid.y * grid.z >= (sizeof(R) == 4 ? 720 : 200) ? roms_sub_launch<R, true>(c, a, grid, s)
                                                                               : roms_sub_launch<R, false>(c, a, grid, s);
+    }
+    if (a.phase != 2 && !roms_by_strips(c)) {
+        for (int mom = 0; mom < 2; ++mom) {
+            cudaError_t e;
+            if (c->nmem > 1) {
+                auto k = a.phase == 0 ? (mom ? kb_roms_point<R, 0, true> : kb_roms_point<R, 0, false>)
+                                      : (mom ? kb_roms_point<R, 1, true> : kb_roms_point<R, 1, false>);
+                e = launch_dep(c, k, c->nbm_pt, 256, 0, s, mt<R>(c), c->bm_pt, a);
+            } else {
+                auto k = a.phase == 0 ? (mom ? k_roms_point<R, 0, true> : k_roms_point<R, 0, false>)
+                                      : (mom ? k_roms_point<R, 1, true> : k_roms_point<R, 1, false>);
+                e = launch_dep(c, k, blocks_for(c->s2, 256), 256, 0, s, geo(c), a);
+            }
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
     }
     if (c->nmem > 1) {
         if (a.phase == 2)

@@ -247,11 +247,8 @@ class Model:
 
     @property
     def loop_launches(self):
-        """Kernel launches of the ROMS-form barotropic loop: of its nfast substeps the first and the
-        last one to six take two, the groups of six between them one each (fused); one more for
-        the averages of substep nfast + 1."""
-        fused = max(0, self.nfast - 2) // 6 * 6
-        return 2 * (self.nfast - fused) + fused + 1
+        """Kernel launches of the ROMS-form barotropic loop on this grid (sf_roms_loop_launches)."""
+        return lib.sf_roms_loop_launches(self.ctx.ptr, self.nfast)
 
     def _roms_loop(self, s, stream):
         W1 = self.W1.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
