@@ -707,6 +707,46 @@ __device__ __forceinline__ void roms_rhs3d_rows(const Geo<R> &g, const R *__rest
     }
 }
 
+// The same at one point and level a thread, every neighbour loaded where it is needed: for basins whose strips
+// would be mostly empty (rule: Ops::roms_rhs3d).
+template <typename R>
+__device__ __forceinline__ void roms_rhs3d_point(const Geo<R> &g, const R *__restrict__ u, const R *__restrict__ v,
+                                                 const R *__restrict__ Hu, const R *__restrict__ Hv,
+                                                 const R *__restrict__ Hz, R *__restrict__ ru, R *__restrict__ rv,
+                                                 const long pl, const int k) {
+    if (pl >= g.s2) return;
+    const int p = (int)pl, I = g.I, j = fdiv(p, g.dI), i = p - j * I;
+    const long o = (long)k * g.s2;
+    const bool in = i >= 1 && i <= I - 2 && j >= 1 && j <= g.J - 2;
+    R tu = R(0), tv = R(0);
+    if (k < g.N && in && (i >= 2 || j >= 2)) {
+        u += o;
+        v += o;
+        Hu += o;
+        Hv += o;
+        Hz += o;
+        const R *fo = g.fomn;
+        const int n = p + I, s = p - I, w = p - 1, e = p + 1;
+        const R cf = rmul(Hz[p], fo[p]), vb = rmul(v[p] + v[n], R(0.5)), ub = rmul(u[p] + u[e], R(0.5));
+        if (i >= 2) {
+            const R ufw = rmul(rmul(Hz[w], fo[w]), rmul(v[w] + v[n - 1], R(0.5)));
+            const R xuw = rmul(rmul(R(0.25), Hu[w] + Hu[p]), u[w] + u[p]);
+            const R es = rmul(rmul(R(0.25), Hv[p] + Hv[w]), u[p] + u[s]);
+            tu = rmul(rfma(cf, vb, ufw), R(0.5)) - (rfma(rmul(R(0.25), Hu[p] + Hu[e]), u[p] + u[e], -xuw) +
+                                                    rfma(rmul(R(0.25), Hv[n] + Hv[n - 1]), u[n] + u[p], -es));
+        }
+        if (j >= 2) {
+            const R vfs = rmul(rmul(Hz[s], fo[s]), rmul(u[s] + u[s + 1], R(0.5)));
+            const R xv = rmul(rmul(R(0.25), Hu[p] + Hu[s]), v[p] + v[w]);
+            const R eps = rmul(rmul(R(0.25), Hv[s] + Hv[p]), v[s] + v[p]);
+            tv = -rmul(rfma(cf, ub, vfs), R(0.5)) - (rfma(rmul(R(0.25), Hu[e] + Hu[s + 1]), v[e] + v[p], -xv) +
+                                                     rfma(rmul(R(0.25), Hv[p] + Hv[n]), v[p] + v[n], -eps));
+        }
+    }
+    ru[o + p] = tu;
+    rv[o + p] = tv;
+}
+
 // Surface and bottom stress on the 3D momentum right-hand side (ROMS's ru includes
 // + sustr om_u on_u at k = N and - bustr om_u on_u at k = 1): ru[N-1] += sustr * area and
 // ru[0] -= rdrag2 ub sqrt(ub^2 + v_u^2) * area at the interior U faces, ub the bottom level's u,
@@ -1085,6 +1125,18 @@ __global__ void __launch_bounds__(32 * kRomsWarps) kb_roms_rhs3d(const Member<R>
                     (by * kRomsWarps + (int)(threadIdx.x >> 5)) * nrows, nrows, (int)blockIdx.y);
 }
 template <typename R>
+__global__ void __launch_bounds__(128) k_roms_rhs3d_point(Geo<R> g, const R *u, const R *v, const R *Hu, const R *Hv,
+                                                          const R *Hz, R *ru, R *rv) {
+    roms_rhs3d_point(g, u, v, Hu, Hv, Hz, ru, rv, tid_flat(), (int)blockIdx.y);
+}
+template <typename R>
+__global__ void __launch_bounds__(128) kb_roms_rhs3d_point(const Member<R> *mt, const int2 *bm, const R *u, const R *v,
+                                                           const R *Hu, const R *Hv, const R *Hz, R *ru, R *rv) {
+    const MemberAt<R> m = member_at(mt, bm, 128);
+    if ((int)blockIdx.y > m.g.N) return;
+    roms_rhs3d_point(m.g, u + m.o3, v + m.o3, Hu + m.o3, Hv + m.o3, Hz + m.oN, ru + m.o3, rv + m.o3, m.p, (int)blockIdx.y);
+}
+template <typename R>
 __global__ void __launch_bounds__(256) k_roms_stress3d(Geo<R> g, const R *u, const R *v, R *ru,
                                                        R *rv, const R *sustr, const R *svstr,
                                                        R rdrag2) {
@@ -1204,7 +1256,16 @@ template <typename R>
 cudaError_t Ops<R>::roms_rhs3d(const sf_ctx *c, const R *u, const R *v, const R *Huon,
                                const R *Hvom, const R *Hz, R *ru, R *rv, cudaStream_t s) {
     const int B = 32 * kRomsWarps;
-    if (c->nmem > 1) {
+    // strips where they hold at least 13 of 29 columns (30 levels, FP32: 12 x 16666 points 69 us by points and 76 by
+    // strips, 14 x 14285 70 and 67, 33 x 6060 73 and 63, 1026 x 514 98 by strips; FP64 98 and 112, 99 and 100, 102 and 93)
+    const bool strips = c->s2 >= 13 * c->roms_strip_rows;
+    if (!strips) {
+        const int levels = (c->nmem > 1 ? c->maxN : c->N) + 1;
+        if (c->nmem > 1)
+            kb_roms_rhs3d_point<R><<<dim3(c->nbm_128, levels), 128, 0, s>>>(mt<R>(c), c->bm_128, u, v, Huon, Hvom, Hz, ru, rv);
+        else
+            k_roms_rhs3d_point<R><<<dim3(blocks_for(c->s2, 128), levels), 128, 0, s>>>(geo(c), u, v, Huon, Hvom, Hz, ru, rv);
+    } else if (c->nmem > 1) {
         kb_roms_rhs3d<R><<<dim3(c->nbm_roms, c->maxN + 1), B, 0, s>>>(mt<R>(c), c->bm_roms, u, v, Huon, Hvom, Hz, ru,
                                                                      rv, c->roms_rows);
     } else {
