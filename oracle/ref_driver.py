@@ -15,6 +15,7 @@ import ctypes
 import math
 import os
 import time
+import unittest
 
 import numpy as np
 
@@ -47,11 +48,17 @@ def available(suffix=""):
     return all(os.path.exists(os.path.join(REF, "libsfref_%s%s.so" % (m, suffix))) for m in SIGS)
 
 
+class ReferenceAbsent(unittest.SkipTest, OSError):
+    """The reference's kernels are not built (its sources are not there): a comparison with them is skipped."""
+
+
 class RefKernels:
     """The reference's kernels from oracle/_ref; suffix "" is the pinned build (-O2, no
     contraction), "_native" the timed build (build_ref.build_native)."""
 
     def __init__(self, omp=1, suffix=""):
+        if not available(suffix):
+            raise ReferenceAbsent("%s/libsfref_*%s.so not built: no reference checkout" % (REF, suffix))
         self.omp = int(omp)
         self.libs = {}
         for mod, fns in SIGS.items():
