@@ -139,7 +139,8 @@ GlsConst<R> gls_const(const sf_gls_params &P, double dt) {
 // sets (a limit on psi in the reference's text) is compared as a length, without one.
 // Blocks per SM: the levels are a chain of divisions and roots, so warps hide the latency, not loads in
 // flight (levels in chunks of 4 at 128 registers: 0.97 and 0.41 ms for the two cases above; one at a
-// time with 10 blocks at 48 registers in FP32, 7 at 72 in FP64: 0.76 and 0.31, 0.68 and 0.30 now; 12 blocks 0.88).
+// time with 10 blocks at 48 registers in FP32, 7 at 72 in FP64, though these spill 16 and 72 bytes a thread: 0.76
+// and 0.31, 0.68 and 0.30 now; 12 blocks 0.88).
 template <typename R>
 constexpr int gls_blocks() { return sizeof(R) == 4 ? 10 : 7; }
 // KEPS: the exponents of k-epsilon, the default model (m = 3/2, n = -1), as constants: the branches on

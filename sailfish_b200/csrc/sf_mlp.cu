@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_fwd(InferW w, long n, cons
 #pragma unroll
         for (int k = 0; k < 32; ++k) v[k] += sbias[l][cb + k];
         float z[32];
-        if (!last) {   // the next product first, its operand's stores beside it
+        if (!last) {   // the next product's operand first; its issuing warp stores its own rows before it
 #pragma unroll
             for (int k = 0; k < 32; ++k) z[k] = act_apply(v[k], ACT);
             store_bf16_32(sA, rl, cb, z);

@@ -81,7 +81,7 @@ __device__ __forceinline__ R roms_new(R u, R Ds, R pmn2, R cdt, R f, R Dn) {
 // Ring nodes of the free surface take the value of the nearest interior node (zero gradient at the
 // closed walls): its owner writes them.
 // Bound: bytes per node and substep 252 in FP32 (80 predictor, 172 corrector of which 80 the
-// averages), 404 in FP64.
+// averages), 424 in FP64.
 template <typename R>
 struct RomsRow {   // a node's inputs of one row
     R z, h, v, om;                       // row j + 1: flux level's zeta and vbar, depth, om_v
@@ -1057,7 +1057,7 @@ constexpr int roms_sub_smem(int H) {
     return (LATE ? 32 * H * (40 + 7 * (int)sizeof(R)) : 0) + (8 * H + 2) * 32 * (int)sizeof(R);
 }
 // Blocks per SM the register cap allows for: LATE in FP32 3 of 384 threads at 56 registers (4 at 40
-// spill: 2050 x 1026 loop 5.10 against 4.35 ms), in FP64 2 at 80; else uncapped.
+// spill: 2050 x 1026 loop 5.10 against 4.35 ms), in FP64 2 at 80 (68 bytes spilled); else uncapped.
 template <typename R, bool LATE>
 constexpr int roms_sub_blocks() { return !LATE ? 1 : (sizeof(R) == 4 ? 3 : 2); }
 template <typename R, int H, bool LATE>
