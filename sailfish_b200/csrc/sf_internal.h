@@ -268,21 +268,25 @@ constexpr int kRomsCols = 29, kRomsWarps = 4;
 constexpr int kSubCols = 27, kSubRows = 12;
 
 // Whether the phases go by strips (two launches a substep), else a point a thread (four).  By strips a row of
-// one costs its 32 lanes whether 29 columns exist or one: about 1.3 ns in FP32 on large grids, 4 in FP64, whose
-// 140 to 180 registers leave 8 warps a SM; by points a node costs 0.06 ns (FP64 0.1) and a substep 13 us at least.
-// us a substep in FP32, strips and points: 29 x 3000 10 and 14, 5 x 9000 19 and 13, 17 x 29411 39 and 33, 20 x 25000 32
-// and 33, 33 x 15151 41 and 33, 1026 x 514 25 and 33, 2050 x 1026 100 and 163; FP64: 17 x 1764 12 and 14, 258 x 130
-// 11 and 14, 29 x 3000 18 and 16, 702 x 402 43 and 29, 1026 x 514 72 and 54, 2050 x 1026 264 and 223.
+// one costs its 32 lanes whether 29 columns exist or one; by points a node costs the same in every basin, but a
+// substep 13 us of launches at least.  us a substep in FP32, strips and points: 29 x 3000 9 and 14, 5 x 9000 18 and 13,
+// 17 x 29411 35 and 32, 20 x 25000 30 and 32, 33 x 15151 36 and 32, 1026 x 514 23 and 33, 2050 x 1026 85 and 156; FP64: 17 x 1764 11
+// and 13, 8 x 3750 19 and 13, 450 x 220 17 and 16, 1501 x 701 95 and 108, 2050 x 1026 184 and 209.  In FP64 the strips'
+// 140 to 180 registers leave 8 warps a SM, and from 2^18 to 2^20 points (4 rows a warp) their few waves end unevenly:
+// 600 x 300 23 and 22, 702 x 402 34 and 26, 1026 x 514 55 and 50 (a loop of 28 substeps, 24 of them fused, 0.69 and 0.66 ms at
+// 702 x 402, but 0.88 and 0.88 at 600 x 300).  An ensemble's point form looks its members up and stays behind
+// (30 members, 1.2e6 points, a loop of 52 substeps: 6.98 and 7.23 ms).
 inline bool roms_by_strips(const sf_ctx *c) {
     const long rows = c->roms_strip_rows, pts = c->s2;
-    if (c->prec == SF_FP32) return rows <= 6000 || pts >= 20 * rows;
-    return rows <= 1800;
+    const bool full = pts >= 20 * rows;
+    if (c->prec == SF_FP32) return rows <= 6000 || full;
+    return rows <= 1800 || (full && (c->nmem > 1 || pts < (1L << 18) || pts >= (1L << 20)));
 }
-// Whether runs of leapfrog substeps go fused: about 13 ns a tile of up to 243 nodes in FP32, 27 in FP64, against the
+// Whether runs of leapfrog substeps go fused: about 12 ns a tile of up to 243 nodes in FP32, 20 in FP64, against the
 // phases' times and the averages.  ms a loop of 28 substeps in FP32, tiles and the phases' better form: 5 x 6000
-// 0.31 and 0.39, 16 x 31250 1.23 and 1.10, 20 x 25000 0.94 and 1.09, 28 x 17857 1.36 and 0.84, 1026 x 514 0.66 and 0.85; FP64:
-// 5 x 6000 0.64 and 0.40, 24 x 20833 1.82 and 1.71 (1.69 with the remainders by points), 40 x 12500 2.17 and 1.70, 1026 x 514
-// 1.66 and 1.82, 2050 x 1026 6.0 and 7.3.
+// 0.28 and 0.38, 16 x 31250 1.14 and 1.03, 20 x 25000 0.88 and 0.94, 28 x 17857 1.30 and 0.73, 1026 x 514 0.63 and 0.76; FP64:
+// 5 x 3000 0.32 and 0.36, 5 x 6000 0.48 and 0.39, 24 x 20833 1.42 and 1.56, 40 x 12500 1.63 and 1.56, 12 x 41666 2.63 and 1.56,
+// 1026 x 514 1.33 and 1.73, 2050 x 1026 4.8 and 5.9.
 inline bool roms_by_tiles(const sf_ctx *c) {
     const long tiles = c->roms_tiles, pts = c->s2;
     return c->prec == SF_FP32 ? 200 * tiles <= pts + 190000 : 225 * tiles <= pts + 100000;

@@ -801,9 +801,9 @@ struct RomsRhs {
 // Levels whose loads the column solve issues together (1003 x 501 x 50, FP32: 2, 4, 6, 8, 12 levels 0.59,
 // 0.59, 0.47, 0.45, 0.53 ms; FP64 4, 6, 8: 1.29, 1.27, 1.33), and the blocks per SM its registers are capped
 // for.  Columns of at most 16 levels (SHORT) have few chunks to issue and little shared memory, so more blocks
-// hide the latency instead: 1026 x 514 x 6 in FP32 112 us with 8 levels and 3 blocks, 79 with 4 and 6, 72 with
-// 2 and 8; FP64 224, 171 and 132 (2 and 10); 16 levels FP32 196, 143, 132, FP64 433, 331, 285; at 24 levels
-// the long form leads (FP32 255 against 282 us).
+// hide the latency instead: 1026 x 514 x 6 in FP32 104 us with 8 levels and 3 blocks, 66 with 2 and 8, FP64 189 and
+// 112 (2 and 10); 16 levels FP32 188 and 128, FP64 361 and 249; at 24 levels the long form leads (FP32 255
+// against 282 us).
 constexpr int kRomsShortN = 16;
 template <typename R>
 constexpr int roms_col_chunk(bool SHORT) { return SHORT ? 2 : (sizeof(R) == 4 ? 8 : 6); }
@@ -1256,11 +1256,14 @@ template <typename R>
 cudaError_t Ops<R>::roms_rhs3d(const sf_ctx *c, const R *u, const R *v, const R *Huon,
                                const R *Hvom, const R *Hz, R *ru, R *rv, cudaStream_t s) {
     const int B = 32 * kRomsWarps;
-    // strips where they hold at least 13 of 29 columns (30 levels, FP32: 12 x 16666 points 69 us by points and 76 by
-    // strips, 14 x 14285 70 and 67, 33 x 6060 73 and 63, 1026 x 514 98 by strips; FP64 98 and 112, 99 and 100, 102 and 93)
-    const bool strips = c->s2 >= 13 * c->roms_strip_rows;
+    // strips where they hold at least 13 of 29 columns, in FP32 with few levels 17 (30 levels, FP32: 12 x 16666
+    // points 69 us
+    // by points and 76 by strips, 14 x 14285 70 and 67, 33 x 6060 73 and 63, 130 x 1538 73 and 46; FP64 98 and 112, 99 and 100,
+    // 102 and 93, 104 and 73; 5 levels, FP32: 16 x 31250 27 and 29, 17 x 29411 27 and 27)
+    const int N = c->nmem > 1 ? c->maxN : c->N;
+    const bool strips = c->s2 >= (sizeof(R) == 4 && N < 10 ? 17 : 13) * c->roms_strip_rows;
     if (!strips) {
-        const int levels = (c->nmem > 1 ? c->maxN : c->N) + 1;
+        const int levels = N + 1;
         if (c->nmem > 1)
             kb_roms_rhs3d_point<R><<<dim3(c->nbm_128, levels), 128, 0, s>>>(mt<R>(c), c->bm_128, u, v, Huon, Hvom, Hz, ru, rv);
         else
