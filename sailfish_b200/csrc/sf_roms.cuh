@@ -1256,10 +1256,9 @@ template <typename R>
 cudaError_t Ops<R>::roms_rhs3d(const sf_ctx *c, const R *u, const R *v, const R *Huon,
                                const R *Hvom, const R *Hz, R *ru, R *rv, cudaStream_t s) {
     const int B = 32 * kRomsWarps;
-    // strips where they hold at least 13 of 29 columns, in FP32 with few levels 17 (30 levels, FP32: 12 x 16666
-    // points 69 us
-    // by points and 76 by strips, 14 x 14285 70 and 67, 33 x 6060 73 and 63, 130 x 1538 73 and 46; FP64 98 and 112, 99 and 100,
-    // 102 and 93, 104 and 73; 5 levels, FP32: 16 x 31250 27 and 29, 17 x 29411 27 and 27)
+    // strips where they hold at least 13 of 29 columns, in FP32 with few levels 17 (us by points and by strips; 30
+    // levels, FP32: 12 x 16666 points 69 and 76, 14 x 14285 70 and 67, 33 x 6060 73 and 63, 130 x 1538 73 and 46; FP64 98 and
+    // 112, 99 and 100, 102 and 93, 104 and 73; 5 levels, FP32: 16 x 31250 27 and 29, 17 x 29411 27 and 27)
     const int N = c->nmem > 1 ? c->maxN : c->N;
     const bool strips = c->s2 >= (sizeof(R) == 4 && N < 10 ? 17 : 13) * c->roms_strip_rows;
     if (!strips) {
