@@ -707,44 +707,45 @@ __device__ __forceinline__ void roms_rhs3d_rows(const Geo<R> &g, const R *__rest
     }
 }
 
-// The same at one point and level a thread, every neighbour loaded where it is needed: for basins whose strips
-// would be mostly empty (rule: Ops::roms_rhs3d).
+// The same, a point a thread, levels k0, k0 + dk, ..., every neighbour loaded where it is needed: for basins whose
+// strips would be mostly empty (rule: Ops::roms_rhs3d).  U and V in branches of their own, loads they share
+// included: in one branch 5 x 200000 points of 5 levels in FP32 took 100 us, so 48.
 template <typename R>
 __device__ __forceinline__ void roms_rhs3d_point(const Geo<R> &g, const R *__restrict__ u, const R *__restrict__ v,
                                                  const R *__restrict__ Hu, const R *__restrict__ Hv,
                                                  const R *__restrict__ Hz, R *__restrict__ ru, R *__restrict__ rv,
-                                                 const long pl, const int k) {
-    if (pl >= g.s2) return;
-    const int p = (int)pl, I = g.I, j = fdiv(p, g.dI), i = p - j * I;
-    const long o = (long)k * g.s2;
-    const bool in = i >= 1 && i <= I - 2 && j >= 1 && j <= g.J - 2;
-    R tu = R(0), tv = R(0);
-    if (k < g.N && in && (i >= 2 || j >= 2)) {
-        u += o;
-        v += o;
-        Hu += o;
-        Hv += o;
-        Hz += o;
-        const R *fo = g.fomn;
-        const int n = p + I, s = p - I, w = p - 1, e = p + 1;
-        const R cf = rmul(Hz[p], fo[p]), vb = rmul(v[p] + v[n], R(0.5)), ub = rmul(u[p] + u[e], R(0.5));
-        if (i >= 2) {
-            const R ufw = rmul(rmul(Hz[w], fo[w]), rmul(v[w] + v[n - 1], R(0.5)));
-            const R xuw = rmul(rmul(R(0.25), Hu[w] + Hu[p]), u[w] + u[p]);
-            const R es = rmul(rmul(R(0.25), Hv[p] + Hv[w]), u[p] + u[s]);
-            tu = rmul(rfma(cf, vb, ufw), R(0.5)) - (rfma(rmul(R(0.25), Hu[p] + Hu[e]), u[p] + u[e], -xuw) +
-                                                    rfma(rmul(R(0.25), Hv[n] + Hv[n - 1]), u[n] + u[p], -es));
+                                                 const long p, const int k0, const int dk) {
+    if (p >= g.s2) return;
+    const int j = fdiv((int)p, g.dI), i = (int)p - j * g.I;
+    const long I = g.I, s2 = g.s2;
+    const int N = g.N;
+    const bool uf = i >= 2 && i <= g.I - 2 && j >= 1 && j <= g.J - 2;
+    const bool vf = j >= 2 && j <= g.J - 2 && i >= 1 && i <= g.I - 2;
+    const R *fo = g.fomn;
+    for (int k = k0; k <= N; k += dk) {
+        const long o = (long)k * s2;
+        R tu = R(0), tv = R(0);
+        if (k < N && uf) {
+            const R *uk = u + o, *vk = v + o, *hu = Hu + o, *hv = Hv + o, *hz = Hz + o;
+            const R cf = rmul(hz[p], fo[p]), vb = rmul(vk[p] + vk[p + I], R(0.5));
+            const R ufw = rmul(rmul(hz[p - 1], fo[p - 1]), rmul(vk[p - 1] + vk[p - 1 + I], R(0.5)));
+            const R xuw = rmul(rmul(R(0.25), hu[p - 1] + hu[p]), uk[p - 1] + uk[p]);
+            const R es = rmul(rmul(R(0.25), hv[p] + hv[p - 1]), uk[p] + uk[p - I]);
+            tu = rmul(rfma(cf, vb, ufw), R(0.5)) - (rfma(rmul(R(0.25), hu[p] + hu[p + 1]), uk[p] + uk[p + 1], -xuw) +
+                                                    rfma(rmul(R(0.25), hv[p + I] + hv[p + I - 1]), uk[p + I] + uk[p], -es));
         }
-        if (j >= 2) {
-            const R vfs = rmul(rmul(Hz[s], fo[s]), rmul(u[s] + u[s + 1], R(0.5)));
-            const R xv = rmul(rmul(R(0.25), Hu[p] + Hu[s]), v[p] + v[w]);
-            const R eps = rmul(rmul(R(0.25), Hv[s] + Hv[p]), v[s] + v[p]);
-            tv = -rmul(rfma(cf, ub, vfs), R(0.5)) - (rfma(rmul(R(0.25), Hu[e] + Hu[s + 1]), v[e] + v[p], -xv) +
-                                                     rfma(rmul(R(0.25), Hv[p] + Hv[n]), v[p] + v[n], -eps));
+        if (k < N && vf) {
+            const R *uk = u + o, *vk = v + o, *hu = Hu + o, *hv = Hv + o, *hz = Hz + o;
+            const R cf = rmul(hz[p], fo[p]), ub = rmul(uk[p] + uk[p + 1], R(0.5));
+            const R vfs = rmul(rmul(hz[p - I], fo[p - I]), rmul(uk[p - I] + uk[p - I + 1], R(0.5)));
+            const R xv = rmul(rmul(R(0.25), hu[p] + hu[p - I]), vk[p] + vk[p - 1]);
+            const R eps = rmul(rmul(R(0.25), hv[p - I] + hv[p]), vk[p - I] + vk[p]);
+            tv = -rmul(rfma(cf, ub, vfs), R(0.5)) - (rfma(rmul(R(0.25), hu[p + 1] + hu[p + 1 - I]), vk[p + 1] + vk[p], -xv) +
+                                                     rfma(rmul(R(0.25), hv[p] + hv[p + I]), vk[p] + vk[p + I], -eps));
         }
+        ru[o + p] = tu;
+        rv[o + p] = tv;
     }
-    ru[o + p] = tu;
-    rv[o + p] = tv;
 }
 
 // Surface and bottom stress on the 3D momentum right-hand side (ROMS's ru includes
@@ -1127,14 +1128,14 @@ __global__ void __launch_bounds__(32 * kRomsWarps) kb_roms_rhs3d(const Member<R>
 template <typename R>
 __global__ void __launch_bounds__(128) k_roms_rhs3d_point(Geo<R> g, const R *u, const R *v, const R *Hu, const R *Hv,
                                                           const R *Hz, R *ru, R *rv) {
-    roms_rhs3d_point(g, u, v, Hu, Hv, Hz, ru, rv, tid_flat(), (int)blockIdx.y);
+    roms_rhs3d_point(g, u, v, Hu, Hv, Hz, ru, rv, tid_flat(), (int)blockIdx.y, (int)gridDim.y);
 }
 template <typename R>
 __global__ void __launch_bounds__(128) kb_roms_rhs3d_point(const Member<R> *mt, const int2 *bm, const R *u, const R *v,
                                                            const R *Hu, const R *Hv, const R *Hz, R *ru, R *rv) {
     const MemberAt<R> m = member_at(mt, bm, 128);
-    if ((int)blockIdx.y > m.g.N) return;
-    roms_rhs3d_point(m.g, u + m.o3, v + m.o3, Hu + m.o3, Hv + m.o3, Hz + m.oN, ru + m.o3, rv + m.o3, m.p, (int)blockIdx.y);
+    roms_rhs3d_point(m.g, u + m.o3, v + m.o3, Hu + m.o3, Hv + m.o3, Hz + m.oN, ru + m.o3, rv + m.o3, m.p, (int)blockIdx.y,
+                     (int)gridDim.y);
 }
 template <typename R>
 __global__ void __launch_bounds__(256) k_roms_stress3d(Geo<R> g, const R *u, const R *v, R *ru,
@@ -1256,13 +1257,16 @@ template <typename R>
 cudaError_t Ops<R>::roms_rhs3d(const sf_ctx *c, const R *u, const R *v, const R *Huon,
                                const R *Hvom, const R *Hz, R *ru, R *rv, cudaStream_t s) {
     const int B = 32 * kRomsWarps;
-    // strips where they hold at least 13 of 29 columns, in FP32 with few levels 17 (us by points and by strips; 30
-    // levels, FP32: 12 x 16666 points 69 and 76, 14 x 14285 70 and 67, 33 x 6060 73 and 63, 130 x 1538 73 and 46; FP64 98 and
-    // 112, 99 and 100, 102 and 93, 104 and 73; 5 levels, FP32: 16 x 31250 27 and 29, 17 x 29411 27 and 27)
+    // Strips where enough of their 29 columns exist.  us by points and by strips, 30 levels, FP32: 14 x 14285 points
+    // 63 and 67, 17 x 11764 62 and 58, 20 x 10000 62 and 52; 5 levels: 17 x 58823 48 and 50, 20 x 50000 48 and 46; FP64,
+    // 30 levels: 12 x 16666 108 and 112, 14 x 14285 108 and 100.  Ensembles, whose strips have the phases' fewer rows,
+    // 32 levels: 22 columns (40 of 66 x 34) FP32 28 and 39, FP64 53 and 58; 27 (12 of 300 x 140) 152 and 129, 228 and 200.
     const int N = c->nmem > 1 ? c->maxN : c->N;
-    const bool strips = c->s2 >= (sizeof(R) == 4 && N < 10 ? 17 : 13) * c->roms_strip_rows;
-    if (!strips) {
-        const int levels = N + 1;
+    const int least = c->nmem > 1 ? 24 : (sizeof(R) == 8 ? 14 : (N < 10 ? 19 : 15));
+    if (c->s2 < least * c->roms_strip_rows) {
+        // by points: the levels of a point over as many threads as small basins need (5 x 6000 points of 30 levels, FP32,
+        // all, 2, 1: 12, 15, 25 us; 5 x 40000 65, 62, 79; 4 members of 8 x 2000, 32 levels, all, 4, 2, 1: 24, 20, 20, 28)
+        const int levels = c->s2 < (1L << 15) ? N + 1 : c->s2 < (1L << 18) ? 4 : 2;
         if (c->nmem > 1)
             kb_roms_rhs3d_point<R><<<dim3(c->nbm_128, levels), 128, 0, s>>>(mt<R>(c), c->bm_128, u, v, Huon, Hvom, Hz, ru, rv);
         else

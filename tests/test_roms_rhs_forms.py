@@ -31,8 +31,9 @@ def _data(g, k):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
-@pytest.mark.parametrize("sizes", [((5, 60, 6), (58, 40, 9)),          # strips; the first alone by points
-                                   ((6, 300, 7), (31, 9, 5)),          # points; the second alone by strips
+@pytest.mark.parametrize("sizes", [((5, 60, 6), (58, 400, 9)),         # strips; the first alone by points
+                                   ((6, 300, 7), (58, 9, 5)),          # points; the second alone by strips
+                                   ((6, 6000, 9), (5, 90, 5)),         # points, four threads a column
                                    ((1100, 960, 5), (90, 31, 6))])     # 8 rows a warp; the first alone 32
 def test_members_equal_single_basins(sizes, prec):
     import torch
@@ -62,7 +63,7 @@ def test_members_equal_single_basins(sizes, prec):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("I,J,N", [(5, 5, 5), (6, 47, 6), (12, 40, 5)])
+@pytest.mark.parametrize("I,J,N", [(5, 5, 5), (6, 47, 6), (12, 40, 5), (6, 6000, 9), (5, 53000, 7)])
 def test_point_form_bit_exact(I, J, N):
     from sailfish_b200 import configs
     from sailfish_b200.model import Model
